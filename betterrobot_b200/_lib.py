@@ -90,6 +90,9 @@ SIGNATURES: dict[str, tuple] = {
                                c_int32, c_void_p, c_void_p, c_void_p]),
     "br_pose_loss_backward": (c_int32, [ctypes.POINTER(BrTree), c_void_p, c_void_p, c_int64, c_void_p, c_int32,
                                         c_void_p, c_void_p, c_int32, c_void_p, c_void_p, c_void_p]),
+    "br_pose_loss_value_grad": (c_int32, [ctypes.POINTER(BrTree), c_void_p, c_int64, c_void_p, c_int32, c_void_p,
+                                          c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_void_p]),
+    "br_scale_rows": (c_int32, [c_void_p, c_void_p, c_int64, c_int64, c_int32, c_void_p, c_void_p]),
 }
 
 _lib = None

@@ -5,11 +5,16 @@
 ``src/better_robot/residuals/pose.py:58-66`` squared and summed over frames.
 In the reference its gradient comes from torch autograd through every SE3 op
 of the FK loop (``src/better_robot/kinematics/forward.py:79-81`` keeps that tape
-on purpose); here ``backward`` is one CUDA kernel (``fk_adjoint.cu``).
+on purpose); here it is the hand-written adjoint of ``fk_adjoint.cu``.
 
-Modes: ``"store"`` saves the world joint placements in the forward pass (read
-back by the backward); ``"recompute"`` saves nothing and re-runs FK in the
-backward; ``"auto"`` stores while ``batch * njoints * 28 B`` fits in the L2 cache.
+A configuration's loss depends on its own q only, so a forward pass whose ``q`` needs a gradient
+computes the loss and each configuration's own gradient together (one walk over the tree instead of
+one per pass); ``backward`` scales that gradient row by row with the incoming one.  Without a
+gradient to compute, the forward evaluates the loss alone.
+
+``mode`` ("store", "recompute" or "auto") chose between saving the joint placements and running the
+kinematics again in the backward.  The one-pass forward needs neither: every mode computes and
+returns the same.
 """
 
 from __future__ import annotations
@@ -22,12 +27,6 @@ from . import _lib
 from .exceptions import ShapeError
 from .kinematics import _validate_q
 from .tree import device_tree
-
-
-def choose_mode(model, batch: int, device) -> str:
-    l2 = torch.cuda.get_device_properties(device).L2_cache_size
-    return "store" if batch * model.njoints * 28 <= l2 else "recompute"
-
 
 _IDS: dict = {}
 
@@ -42,6 +41,30 @@ def _ids(frame_ids: tuple):
     return arr
 
 
+def path_slots(arrays, frame_ids: tuple) -> int:
+    """Most joints on one root-to-leaf path that hold a waiting wrench in the adjoint's walk: in the tree
+    pruned to the frames' ancestors, those with a child and a frame of their own or a second child.
+    Kept with the tree table, per frame set."""
+    n = arrays.path_slots.get(frame_ids)
+    if n is None:
+        framed = {int(arrays.frame_parent[f]) for f in frame_ids}
+        support = [int(x) for x in arrays.support]
+        need = 0
+        for j in framed:
+            need |= support[j]
+        children = [0] * arrays.nj
+        for j in range(1, arrays.nj):
+            if need >> j & 1 and arrays.parent[j] >= 0:
+                children[arrays.parent[j]] += 1
+        stored = sum(1 << j for j in range(arrays.nj)
+                     if children[j] >= 2 or (children[j] == 1 and j in framed))
+        n = max(bin(support[j] & stored).count("1") for j in framed)
+        if len(arrays.path_slots) >= 256:
+            arrays.path_slots.clear()
+        arrays.path_slots[frame_ids] = n
+    return n
+
+
 def _on_device(device, fn) -> None:
     """Run ``fn(stream)`` with ``device`` current (no context switch when it already is)."""
     if device.index == torch.cuda.current_device():
@@ -51,38 +74,39 @@ def _on_device(device, fn) -> None:
             fn(torch.cuda.current_stream().cuda_stream)
 
 
+def _loss_only(model, q, frame_ids, targets, weights):
+    loss = torch.empty(q.shape[0], device=q.device, dtype=torch.float32)
+    _on_device(q.device, lambda s: _lib.call(
+        "br_pose_loss", device_tree(model, q.device).ptr, q.data_ptr(), q.shape[0], _ids(frame_ids), len(frame_ids),
+        targets.data_ptr(), weights.data_ptr(), int(weights.dim() == 2), loss.data_ptr(), None, s))
+    return loss
+
+
 class _PoseLoss(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, targets, weights, model, frame_ids, mode):
-        B = q.shape[0]
-        dt = device_tree(model, q.device)
-        ids = _ids(frame_ids)
-        loss = torch.empty(B, device=q.device, dtype=torch.float32)
-        oMi = torch.empty(B, model.njoints, 7, device=q.device) if mode == "store" else None
-        per_cfg = int(weights.dim() == 2)
+    def forward(ctx, q, targets, weights, model, frame_ids, want_grad):
+        if not want_grad:
+            return _loss_only(model, q, frame_ids, targets, weights)
+        loss = torch.empty(q.shape[0], device=q.device, dtype=torch.float32)
+        unit = torch.empty_like(q)
         _on_device(q.device, lambda s: _lib.call(
-            "br_pose_loss", dt.ptr, q.data_ptr(), B, ids, len(frame_ids), targets.data_ptr(), weights.data_ptr(),
-            per_cfg, loss.data_ptr(), oMi.data_ptr() if oMi is not None else None, s))
-        ctx.model, ctx.frame_ids, ctx.per_cfg = model, frame_ids, per_cfg
-        if oMi is not None:
-            ctx.save_for_backward(q, targets, weights, oMi)
-        else:
-            ctx.save_for_backward(q, targets, weights)
+            "br_pose_loss_value_grad", device_tree(model, q.device).ptr, q.data_ptr(), q.shape[0], _ids(frame_ids),
+            len(frame_ids), targets.data_ptr(), weights.data_ptr(), int(weights.dim() == 2),
+            path_slots(device_tree(model, q.device).arrays, frame_ids), loss.data_ptr(), unit.data_ptr(), s))
+        # the inputs too: changing one in place before the backward stays an error
+        ctx.save_for_backward(q, targets, weights, unit)
         return loss
 
     @staticmethod
     def backward(ctx, grad_loss):
-        saved = ctx.saved_tensors
-        q, targets, weights = saved[:3]
-        oMi = saved[3] if len(saved) > 3 else None
-        g = grad_loss.contiguous().float()
-        grad_q = torch.empty_like(q)
-        dt = device_tree(ctx.model, q.device)
-        ids = _ids(ctx.frame_ids)
-        _on_device(q.device, lambda s: _lib.call(
-            "br_pose_loss_backward", dt.ptr, q.data_ptr(), oMi.data_ptr() if oMi is not None else None,
-            q.shape[0], ids, len(ctx.frame_ids), targets.data_ptr(), weights.data_ptr(), ctx.per_cfg,
-            g.data_ptr(), grad_q.data_ptr(), s))
+        unit = ctx.saved_tensors[3]
+        g = grad_loss if grad_loss.dtype == torch.float32 else grad_loss.float()
+        if g.stride(0) not in (0, 1):
+            g = g.contiguous()
+        grad_q = torch.empty_like(unit)
+        _on_device(unit.device, lambda s: _lib.call(
+            "br_scale_rows", unit.data_ptr(), g.data_ptr(), g.stride(0), unit.shape[0], unit.shape[1],
+            grad_q.data_ptr(), s))
         return grad_q, None, None, None, None, None
 
 
@@ -103,9 +127,8 @@ def pose_loss(model, q: torch.Tensor, frame_ids: Sequence[int], targets: torch.T
         raise ShapeError(f"targets must be ({B}, {F}, 7), got {tuple(targets.shape)}")
     if weights.shape not in ((F,), (B, F)):
         raise ShapeError(f"weights must be ({F},) or ({B}, {F}), got {tuple(weights.shape)}")
-    if mode == "auto":
-        mode = choose_mode(model, B, q.device)
-    if mode not in ("store", "recompute"):
+    if mode not in ("store", "recompute", "auto"):
         raise ValueError(f"mode must be 'store', 'recompute' or 'auto', got {mode!r}")
+    want_grad = torch.is_grad_enabled() and (q.requires_grad or targets.requires_grad or weights.requires_grad)
     return _PoseLoss.apply(q.contiguous(), targets.contiguous().float(), weights.contiguous().float(), model,
-                           frame_ids, mode)
+                           frame_ids, want_grad)

@@ -66,6 +66,7 @@ struct DeviceInfo {
   int device = -1;
   int sms = 0;
   int max_smem_optin = 0;
+  int smem_per_sm = 0;
   size_t l2_bytes = 0;
 };
 
@@ -84,7 +85,7 @@ struct FastDiv {
 
 const DeviceInfo& device_info();
 
-inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+__host__ __device__ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline bool aligned4(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; }
 
 int validate_tree(const br_tree_t* t);

@@ -210,6 +210,84 @@ __device__ __forceinline__ void se3_log(const Pose& T, float3& v, float3& w) {
   v = axpy(c, cross(w, wt), axpy(-0.5f, wt, T.t));
 }
 
+// xi = (v, w) = log(T) together with (gl, ga) = Jr^-1(xi)^T xi (jr_inv_T_xi above): the two maps
+// share the half angle a = th/2, 1/(s a) and the V^-1 coefficient, and sin(th/2), cos(th/2) are
+// |q_xyz| and |q_w| of the (normalised) quaternion, so no trigonometric call is made.
+__device__ __forceinline__ void se3_log_grad(const Pose& T, float3& v, float3& w, float3& gl, float3& ga) {
+  float4 q = T.q;
+  if (q.w < 0.f) q = make_float4(-q.x, -q.y, -q.z, -q.w);
+  const float s2 = q.x * q.x + q.y * q.y + q.z * q.z;
+  const float qw = fminf(q.w, 1.f);
+  float factor, c, th2, it, s;
+  if (s2 < 0.25e-8f) {
+    factor = 2.f + s2 * (2.f / 3.f);
+    th2 = factor * factor * s2;
+    c = vinv_series(th2);
+    it = s = 0.f;
+  } else {
+    s = s2 * rsqrtf(s2);
+    const float a = atan_q1(s, qw);
+    const float r = __fdividef(1.f, s * a);
+    factor = 2.f * (a * a) * r;
+    th2 = 4.f * (a * a);
+    c = th2 < 1.f ? vinv_series(th2) : 0.25f * r * fmaf(s2, r, -qw);
+    it = 0.5f * s * r;                             // 1 / th
+  }
+  w = f3(factor * q.x, factor * q.y, factor * q.z);
+  float c2, c3, c4;
+  if (th2 < 2.f) {
+    c2 = fmaf(th2, fmaf(th2, fmaf(th2, fmaf(th2, 1.f / 39916800.f, -1.f / 362880.f), 1.f / 5040.f), -1.f / 120.f),
+              1.f / 6.f);
+    c3 = fmaf(th2, fmaf(th2, fmaf(th2, fmaf(th2, 1.f / 479001600.f, -1.f / 3628800.f), 1.f / 40320.f),
+                   -1.f / 720.f), 1.f / 24.f);
+    c4 = fmaf(th2, fmaf(th2, fmaf(th2, fmaf(th2, 1.f / 1245404160.f, -1.f / 9979200.f), 1.f / 120960.f),
+                   -1.f / 2520.f), 1.f / 120.f);
+  } else {
+    const float n = rsqrtf(fmaf(q.w, q.w, s2));    // unit half-angle pair, also for a quaternion off the sphere
+    const float sh = s * n, ch = q.w * n;
+    const float sn = 2.f * sh * ch, co = fmaf(-2.f * sh, sh, 1.f);
+    const float th = th2 * it, it2 = it * it;
+    c2 = (th - sn) * (it2 * it);
+    c3 = 0.5f * (th2 + 2.f * co - 2.f) * (it2 * it2);
+    c4 = 0.5f * (2.f * th - 3.f * sn + th * co) * (it2 * it2 * it);
+  }
+  const float3 wt = cross(w, T.t);
+  v = axpy(c, cross(w, wt), axpy(-0.5f, wt, T.t));
+  const float3 wv = cross(w, v);
+  gl = axpy(c, cross(w, wv), axpy(-0.5f, wv, v));
+  const float3 a1 = cross(w, gl), a2 = cross(w, a1);
+  const float3 b0 = cross(v, gl), b1 = cross(v, a1), b2 = cross(v, a2);
+  const float3 wb0 = cross(w, b0), wwb0 = cross(w, wb0), wb1 = cross(w, b1), wwb1 = cross(w, wb1);
+  const float3 wb2 = cross(w, b2);
+  float3 x = scale(b0, 0.5f);
+  x = axpy(c2, add(add(wb0, b1), wb1), x);
+  x = axpy(c3, add(add(wwb0, b2), scale(wb1, -3.f)), x);
+  x = axpy(c4, add(wb2, wwb1), x);
+  const float3 wx = cross(w, x);
+  ga = sub(w, axpy(c, cross(w, wx), axpy(-0.5f, wx, x)));
+}
+
+// sin(x / 2), cos(x / 2) for |x| <= kSincosHalfMax, without a branch (independent evaluations
+// interleave): x / 2 - n pi/2 with n = round(x / pi) by three multiply-adds (Cody and Waite's split of
+// pi/2), then polynomials in u = r^2 fitted here on [-pi/4, pi/4] (iteratively reweighted least squares
+// towards the minimax: 3.6e-9 for sin, 9.6e-11 for cos in exact arithmetic) and the quadrant's swap and
+// signs.  Within 9.3e-8 of the exact values over the range (sincosf: 7e-8).
+constexpr float kSincosHalfMax = 30000.f;
+__device__ __forceinline__ void sincos_half(float x, float& s, float& c) {
+  const float t = fmaf(x, 0.318309886f, 12582912.f);        // 1.5 2^23: the integer in the low bits
+  const int n = __float_as_int(t);
+  const float fn = t - 12582912.f;
+  float r = fmaf(fn, -1.57079637f, 0.5f * x);
+  r = fmaf(fn, 4.37113883e-8f, r);
+  r = fmaf(fn, 1.71512451e-15f, r);
+  const float u = r * r;
+  const float sp = fmaf(fmaf(fmaf(-0.000195169778f, u, 0.00833217613f), u, -0.166666552f), u * r, r);
+  const float cp = fmaf(fmaf(fmaf(2.44380899e-5f, u, -0.00138873642f), u, 0.0416666456f), u * u, fmaf(u, -0.5f, 1.f));
+  const float a = (n & 1) ? cp : sp, b = (n & 1) ? sp : cp;
+  s = __int_as_float(__float_as_int(a) ^ ((n & 2) << 30));
+  c = __int_as_float(__float_as_int(b) ^ (((n + 1) & 2) << 30));
+}
+
 // so3_exp (_torch_native_backend.py:144-159)
 __device__ __forceinline__ float4 so3_exp(float3 w) {
   const float th2 = dot(w, w);

@@ -437,6 +437,7 @@ const DeviceInfo& device_info() {
     cudaGetDeviceProperties(&prop, dev);
     d.sms = prop.multiProcessorCount;
     d.max_smem_optin = (int)prop.sharedMemPerBlockOptin;
+    d.smem_per_sm = (int)prop.sharedMemPerMultiprocessor;
     d.l2_bytes = prop.l2CacheSize;
     d.device = dev;
   }

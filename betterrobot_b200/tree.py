@@ -138,6 +138,7 @@ class TreeArrays:
         self.dof_depth = int(ddep.max()) + 1 if nv else 1
         self.lower = _np(model.lower_pos_limit).astype(np.float32)
         self.upper = _np(model.upper_pos_limit).astype(np.float32)
+        self.path_slots: dict = {}  # per frame set (adjoint.path_slots)
 
     def sections(self):
         return [("parent", self.parent), ("jtype", self.jtype), ("idx_q", self.idx_q), ("idx_v", self.idx_v),

@@ -290,6 +290,24 @@ BR_API int br_pose_loss_backward(const br_tree_t* tree, const float* q, const fl
                                  const float* weights, int32_t weights_per_config, const float* grad_loss,
                                  float* grad_q, void* stream);
 
+/*
+ * Loss and gradient in one pass: loss[b] as br_pose_loss, unit_grad[b, :] = dloss[b]/dq as
+ * br_pose_loss_backward with grad_loss = 1.  The loss of a configuration depends on its own q only,
+ * so the gradient for any grad_loss is unit_grad scaled row by row (br_scale_rows).
+ * path_slots: if known, an upper bound on the joints of one root-to-leaf path of the tree pruned to the
+ * frames' ancestors that have a child there and also a frame or a second child (fewer reserved shared
+ * memory, more warps); -1: not known.  Given too small, the results are NaN.
+ */
+BR_API int br_pose_loss_value_grad(const br_tree_t* tree, const float* q, int64_t batch, const int32_t* frame_ids,
+                                   int32_t n_frames, const float* targets, const float* weights,
+                                   int32_t weights_per_config, int32_t path_slots, float* loss, float* unit_grad,
+                                   void* stream);
+
+/* out[i, :] = rows[i, :] * scale[i * scale_stride] for n contiguous rows of `width` floats (stride 0:
+ * one scale for every row). */
+BR_API int br_scale_rows(const float* rows, const float* scale, int64_t scale_stride, int64_t n, int32_t width,
+                         float* out, void* stream);
+
 /* ==== batched trajectory optimisation (Gauss-Newton / LM) ================ */
 #define BR_MAX_TRAJ_KNOTS 128
 #define BR_MAX_TRAJ_NV 64
