@@ -631,53 +631,7 @@ __device__ __forceinline__ double3 dapply_poly(const double3& w, double b0, doub
   return dadd(dadd(dscale(x, b0), dscale(wx, b1)), dscale(dcross(w, wx), b2));
 }
 
-template <int N>
-__device__ __forceinline__ DJrInv djr_inv_se3(double3 v, double3 w) {
-  double ck[N + 1];
-  {
-    double f = 1.0;
-#pragma unroll
-    for (int k = 0; k <= N; ++k) {
-      f /= (double)(k + 1);
-      ck[k] = (k & 1) ? -f : f;
-    }
-  }
-  const double th2 = ddot(w, w);
-  double a0 = ck[N], a1 = 0.0, a2 = 0.0;
-  double B[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-  for (int k = N - 1; k >= 0; --k) {
-    double nB[9];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const double3 bc = d3(B[c], B[3 + c], B[6 + c]);
-      const double3 e = d3(c == 0 ? 1.0 : 0.0, c == 1 ? 1.0 : 0.0, c == 2 ? 1.0 : 0.0);
-      const double3 ac = dapply_poly(w, a0, a1, a2, e);
-      const double3 r = dadd(dcross(w, bc), dcross(v, ac));
-      nB[c] = r.x; nB[3 + c] = r.y; nB[6 + c] = r.z;
-    }
-#pragma unroll
-    for (int i = 0; i < 9; ++i) B[i] = nB[i];
-    const double na1 = a0 - th2 * a2;
-    a2 = a1;
-    a1 = na1;
-    a0 = ck[k];
-  }
-  DJrInv J;
-  J.w = w;
-  const double b0 = 1.0 / a0;
-  const double m = a0 - th2 * a2;
-  const double r0 = -a1 * b0, r1 = -a2 * b0;
-  const double idet = 1.0 / (m * m + th2 * a1 * a1);
-  J.b0 = b0;
-  J.b1 = (r0 * m + th2 * a1 * r1) * idet;
-  J.b2 = (m * r1 - a1 * r0) * idet;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) J.B[i] = B[i];
-  return J;
-}
-
-// One column of djr_inv_se3<N> (see jr_inv_se3_col).
+// One column of the inverse of the N-term series (see jr_inv_se3_col).
 template <int N>
 __device__ __forceinline__ double3 djr_inv_se3_col(double3 v, double3 w, int c, double& b0, double& b1, double& b2) {
   double ck[N + 1];
@@ -709,6 +663,44 @@ __device__ __forceinline__ double3 djr_inv_se3_col(double3 v, double3 w, int c, 
   b1 = (r0 * m + th2 * a1 * r1) * idet;
   b2 = (m * r1 - a1 * r0) * idet;
   return bc;
+}
+
+// All three columns with the series rolled (the coefficients by recurrence): for a long series that runs
+// once, where unrolled code would only push other code out of the instruction cache.
+template <int N>
+__device__ __forceinline__ DJrInv djr_inv_se3_rolled(double3 v, double3 w) {
+  double c = 1.0;                                  // (-1)^N / (N + 1)!
+  for (int k = 2; k <= N + 1; ++k) c /= -(double)k;
+  const double th2 = ddot(w, w);
+  double a0 = c, a1 = 0.0, a2 = 0.0;
+  double B[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+  for (int k = N - 1; k >= 0; --k) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double3 e = d3(i == 0 ? 1.0 : 0.0, i == 1 ? 1.0 : 0.0, i == 2 ? 1.0 : 0.0);
+      const double3 ac = dapply_poly(w, a0, a1, a2, e);
+      const double3 r = dadd(dcross(w, d3(B[i], B[3 + i], B[6 + i])), dcross(v, ac));
+      B[i] = r.x; B[3 + i] = r.y; B[6 + i] = r.z;
+    }
+    const double na1 = a0 - th2 * a2;
+    a2 = a1;
+    a1 = na1;
+    c *= -(double)(k + 2);
+    a0 = c;
+  }
+  DJrInv J;
+  J.w = w;
+  const double b0 = 1.0 / a0;
+  const double m = a0 - th2 * a2;
+  const double r0 = -a1 * b0, r1 = -a2 * b0;
+  const double idet = 1.0 / (m * m + th2 * a1 * a1);
+  J.b0 = b0;
+  J.b1 = (r0 * m + th2 * a1 * r1) * idet;
+  J.b2 = (m * r1 - a1 * r0) * idet;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) J.B[i] = B[i];
+  return J;
 }
 
 __device__ __forceinline__ void djr_inv_apply(const DJrInv& J, double3 xl, double3 xa, double3& ol, double3& oa) {

@@ -1,4 +1,4 @@
-// traj_gn.cu — batched trajectory optimisation (Gauss-Newton / LM), one warp per
+// traj_gn.cu — batched trajectory optimisation (Gauss-Newton / LM), one CTA per
 // trajectory, Newton step in nested-dissection order.
 //
 // Reference: solve_trajopt with knot parameterisation
@@ -16,15 +16,31 @@
 // t, t+1, t+2 of the same DOF, limits / reference / damping are diagonal.  So H is
 // nv independent scalar PENTA-diagonal T x T matrices (one per DOF) plus the dense
 // nv x nv pose blocks at knots 0 and T-1.  The kernel solves it in nested-dissection
-// order: the interior knots 1..T-2 of each DOF first — lane i runs the banded
-// LDL^T of DOF i and three solves (right-hand side and the two columns that tie the
-// interior to knots 0 and T-1) — leaving a 2nv x 2nv Schur complement on the
+// order: the interior knots 1..T-2 of each DOF first — two threads per DOF run the
+// banded L D L^T from both ends with the right-hand side and the columns that tie the
+// interior to knots 0 and T-1 — leaving a 2nv x 2nv Schur complement on the
 // boundary knots,
 //   S = H_bb - H_bI P^-1 H_Ib,   P = blockdiag_i(P_i) the per-DOF interior bands,
-// which the warp factors with a dense Cholesky; the interior step follows by one
-// update.  This is the exact Cholesky of a symmetric permutation of H (no
-// approximation): O(T nv) sequential work per iteration instead of the O(T nv^3) of
-// a block-banded factorization or the O((T nv)^3) of the dense one.
+// which the block factors in panels of eight columns with its right-hand side as one
+// more row; the interior step follows by one more band solve.  This is the exact
+// factorization of a symmetric permutation of H (no approximation): O(T nv) sequential
+// work per iteration instead of the O(T nv^3) of a block-banded factorization or the
+// O((T nv)^3) of the dense one.
+//
+// Bound by the latency of one CTA's dependent steps (a launch lasts as long as its slowest
+// trajectory).  Cycles per Gauss-Newton iteration, chain of 7 at 64 knots / humanoid at 40 knots:
+//   band factorization 14.7 k / 12.3 k -> 4.7 k / 5.4 k  (one multiply-add and one reciprocal between
+//     pivots; the diagonal and the next row's operands loaded off the chain; no early exit, unrolled)
+//   boundary factorization and substitutions 13.5 k / 187 k -> 4.8 k / 37 k  (was one column at a time,
+//     three block barriers and an index decode per entry each)
+//   boundary assembly 1.2 k / 13.9 k -> 2.6 k / 6.6 k  (now with the pose J^T J that the build made)
+//   back substitution 7.5 k / 5.5 k -> 3.7 k / 3.2 k
+//   gradient 6.5 k / 16 k -> 4.7 k / 6.2 k  (Jr^-1 series: three lanes, a column each)
+//   retraction and cost 6.6 k / 68 k -> 6.3 k / 16 k  (the float64 logs and exps of a free-flyer base
+//     one lane each, where every warp of a pass held a single one)
+// 256 x 64-knot chain trajectories 665 -> 362 us, 33 x 40-knot humanoid ones 1,332 -> 315 us.
+// Cyclic reduction of the bands (one warp per DOF, log2 levels of 2 x 2 blocks) measured slower than the
+// two-ended recurrence at every size (chain, 64 knots: 148 against 127 us for six iterations).
 //
 // Precision: the normal matrix has condition ~1e8 (acceleration stiffness
 // (w/dt^2)^2 against a 1e-6 regularisation).  A float32 factorization fails there,
@@ -65,10 +81,10 @@ struct TrajParams {
 
 struct TrajLayout {
   // doubles
-  int x, xn, dd, dr, g, delta, bl1, bdi, Sb, sdi, rb, zb, Jg, Js, rg, rs, jtjg, jtjs, pA, pB, red;
+  int x, xn, dd, dr, g, delta, bl1, bdi, Sb, sdi, sd, zb, schur, Jg, Js, rg, rs, pA, pB, red;
   int total_doubles;
   // 4-byte arrays (offsets in doubles)
-  int xref, parent, jtype, idxq, idxv, dofq, cjoint, ckind, axis, place, caxis, anc, lower, upper;
+  int xref, parent, jtype, idxq, idxv, dofq, heavy, cjoint, ckind, axis, place, caxis, anc, lower, upper;
   int total;
   __host__ __device__ TrajLayout(int nj, int nq, int nv, int T, bool floating) {
     int o = 0;
@@ -81,15 +97,17 @@ struct TrajLayout {
     // per-DOF interior band factors (index p * nv + i, p = knot - 1): L[p][p-1] and 1 / D[p]
     // (L[p][p-2] = c^2 / D[p-2] is rebuilt from 1 / D)
     bl1 = take(T * nv); bdi = take(T * nv);
-    Sb = take(nb * (nb + 1) / 2); sdi = take(nb); rb = take(nb); zb = take(nb);  // boundary Schur complement
+    // boundary Schur complement, packed lower, its right-hand side as row nb; 1 / pivot, pivot, solution
+    Sb = take((nb + 1) * (nb + 2) / 2); sdi = take(nb); sd = take(nb); zb = take(nb);
+    schur = take(5 * nv);                     // per DOF: h0' P^-1 h0, h0' P^-1 hT, hT' P^-1 hT, h0' P^-1 y, hT' P^-1 y
     Jg = take(6 * nv); Js = take(6 * nv); rg = take(8); rs = take(8);
-    jtjg = take(nv * (nv + 1) / 2); jtjs = take(nv * (nv + 1) / 2);              // packed lower
     pA = take(16 * nj); pB = take(16 * nj);   // FK buffers of the two pose terms (goal, start)
     red = take(32);                           // per-warp partial sums of the block reductions
     total_doubles = o;
     auto take4 = [&](int n) { int r = o; o += ((n + 3) & ~3) / 2; return r; };
     xref = take4(T * nq);                     // float32, as given
     parent = take4(nj); jtype = take4(nj); idxq = take4(nj); idxv = take4(nj); dofq = take4(nv);
+    heavy = take4(nj + 1);
     cjoint = take4(nv); ckind = take4(nv);
     axis = take4(4 * nj); place = take4(8 * nj); caxis = take4(4 * nv); anc = take4(8 * nj);
     lower = take4(nq); upper = take4(nq);
@@ -105,23 +123,15 @@ __device__ __forceinline__ void std8d(double* p, const DPose& P) {
   p[4] = P.q.x; p[5] = P.q.y; p[6] = P.q.z; p[7] = P.q.w;
 }
 
-// 1 / d for d > 0 (a pivot): the hardware reciprocal estimate refined by two Newton steps
-// r <- r + r (1 - d r), each of which squares the relative error (~2^-23 -> 2^-46 -> below
-// double rounding); within an ulp or two of 1.0 / d at a fraction of the division's latency.
+// 1 / d for d > 0 (a pivot): the hardware reciprocal estimate r (relative error below 2^-20) refined by
+// one third-order step r <- r + r (e + e^2), e = 1 - d r, which leaves e^3 < 2^-60: within an ulp or two
+// of 1.0 / d in three dependent operations.  Every dependent float64 operation of a recurrence costs
+// about 25 cycles of its single warp's time, so the recurrences below are written to have few of them.
 __device__ __forceinline__ double fast_rcp(double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  double e = fma(-d, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-d, r, 1.0);
-  return fma(r, e, r);
-}
-// 1 / sqrt(x) for x > 0: estimate + two Newton steps y <- y (3 - x y^2) / 2
-__device__ __forceinline__ double fast_rsqrt(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = y * fma(-0.5 * x * y, y, 1.5);
-  return y * fma(-0.5 * x * y, y, 1.5);
+  const double e = fma(-d, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
 
 // packed lower-triangle index p -> (a, b), b <= a, p = a (a + 1) / 2 + b: approximate square
@@ -134,20 +144,22 @@ __device__ __forceinline__ int2 tri_decode(int p) {
 }
 __device__ __forceinline__ int tri_at(int r, int c) { return r * (r + 1) / 2 + c; }  // r >= c
 
-// Threads per trajectory: the per-DOF interior chains take one thread each (nv <= 64),
-// the two pose terms one warp each, everything else strides over the block.
-constexpr int kTrajThreads = 128;
+// Threads per trajectory (kNT): the per-DOF interior chains take two threads each (nv <= 64), the two
+// pose terms one warp each, everything else strides over the block.  256 threads when an SM holds only
+// one trajectory anyway (few trajectories, or a working set above half its shared memory), else 128
+// (64 trajectories of 64 knots, six iterations, 256 against 128 threads: chain of 7 94 against 100 us,
+// 20 DOFs 144 / 160, humanoid 250 / 280; with more trajectories than SMs two CTAs of 128 run at once).
 
 // kManifold: the tree has joints whose configuration is not their tangent coordinates
 // (free-flyer, spherical, planar, unbounded revolute): knot differences and the retraction go
 // through Model.difference / Model.integrate; otherwise they are q1 - q0 and q + v.
-template <bool kManifold>
-__global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams P) {
+template <bool kManifold, int kNT>
+__global__ void __launch_bounds__(kNT, 256 / kNT) traj_gn_kernel(const TrajParams P) {
   extern __shared__ __align__(16) double sm[];
   const br_tree_t& tree = P.tree;
   const int nj = tree.njoints, nq = tree.nq, nv = tree.nv, T = P.T;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NT = kTrajThreads, NW = kTrajThreads / kWarp;
+  constexpr int NT = kNT, NW = kNT / kWarp;
   const int64_t traj = blockIdx.x;
   if (traj >= P.n) return;
   const TrajLayout L(nj, nq, nv, T, kManifold);
@@ -159,14 +171,13 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
   double* bdi = sm + L.bdi;
   double* Sb = sm + L.Sb;
   double* sdi = sm + L.sdi;
-  double* rb = sm + L.rb;
+  double* sd = sm + L.sd;
   double* zb = sm + L.zb;
+  double* schur = sm + L.schur;
   double* Jg = sm + L.Jg;
   double* Js = sm + L.Js;
   double* rg = sm + L.rg;
   double* rs = sm + L.rs;
-  double* jtjg = sm + L.jtjg;
-  double* jtjs = sm + L.jtjs;
   double* pA = sm + L.pA;
   double* pB = sm + L.pB;
   double* red = sm + L.red;
@@ -176,6 +187,7 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
   int* idxq = reinterpret_cast<int*>(sm + L.idxq);
   int* idxv = reinterpret_cast<int*>(sm + L.idxv);
   int* dofq = reinterpret_cast<int*>(sm + L.dofq);  // q slot of a DOF with a position limit, else -1
+  int* heavy = reinterpret_cast<int*>(sm + L.heavy);  // [0] their count, then the joints that are not q + v
   double* dd = sm + L.dd;
   double* dr = sm + L.dr;
   int* cjoint = reinterpret_cast<int*>(sm + L.cjoint);
@@ -194,7 +206,7 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
   const bool has_start = P.start != nullptr && S.w_start > 0.f;
   const bool has_goal = S.w_goal > 0.f;
   const int n = T * nv, nqT = T * nq, nb = 2 * nv;
-  const FastDiv divj(nj > 0 ? nj : 1), divv(nv > 0 ? nv : 1), divq(nq > 0 ? nq : 1);
+  const FastDiv divv(nv > 0 ? nv : 1), divq(nq > 0 ? nq : 1);
 
   for (int j = tid; j < nj; j += NT) {
     parent[j] = tree.parent[j];
@@ -218,6 +230,12 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
     const int jt = jtype[j];
     const bool vec = joint_is_vector(jt);
     for (int k = 0; k < joint_nv(jt); ++k) dofq[idxv[j] + k] = vec ? idxq[j] + k : -1;
+  }
+  if (kManifold && tid == 0) {
+    int nh = 0;
+    for (int j = 0; j < nj; ++j)
+      if (joint_nv(jtype[j]) && !joint_is_vector(jtype[j])) heavy[++nh] = j;
+    heavy[0] = nh;
   }
   const float* x0 = P.x0 + traj * (int64_t)nqT;
   const float* xr = (P.xref ? P.xref : P.x0) + traj * (int64_t)nqT;
@@ -307,7 +325,16 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
           if (lane == 0) { r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = w.x; r[4] = w.y; r[5] = w.z; }
         }
         if (want_J) {
-          const DJrInv Jr = djr_inv_se3<9>(v, w);
+          // the series' three B columns on three lanes
+          DJrInv Jr;
+          Jr.w = w;
+          const double3 bc = djr_inv_se3_col<9>(v, w, lane < 3 ? lane : 0, Jr.b0, Jr.b1, Jr.b2);
+#pragma unroll
+          for (int c3 = 0; c3 < 3; ++c3) {
+            Jr.B[c3] = __shfl_sync(0xffffffffu, bc.x, c3);
+            Jr.B[3 + c3] = __shfl_sync(0xffffffffu, bc.y, c3);
+            Jr.B[6 + c3] = __shfl_sync(0xffffffffu, bc.z, c3);
+          }
           const double4 qc = dqconj(Tee.q);
           for (int k = lane; k < nv; k += kWarp) {
             double3 ol = d3(0, 0, 0), oa = d3(0, 0, 0);
@@ -337,13 +364,14 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
   // (model.py:176-190): free-flyer log(q_a^-1 q_b) (free_flyer.py:53-57), spherical
   // log(normalize(q_a^-1 q_b)) (spherical.py:58-62), angle differences of atan2 for the
   // unbounded revolute and planar joints (revolute.py:233-237, planar.py:70-76)
+  // The joints with a log or an arctangent take one lane per (joint, pair): by (pair, joint) in joint
+  // order every warp held one such lane and 31 subtractions (humanoid, 40 knots: 79 logs in 20 passes
+  // of the block, 68 k cycles per cost with the retraction; now one pass).
   auto knot_differences = [&](const double* xs) {
-    const int npair = 2 * T - 1;
-    for (int e = tid; e < npair * nj; e += NT) {
-      const int pi = divj.div(e), j = e - pi * nj;
-      const int jt = jtype[j], nvj = joint_nv(jt);
-      if (nvj == 0) continue;
-      const int iq = idxq[j], iv = idxv[j];
+    const int npair = 2 * T - 1, nh = heavy[0];
+    for (int e = tid; e < npair * nh; e += NT) {
+      const int hj = e / npair, pi = e - hj * npair, j = heavy[1 + hj];
+      const int jt = jtype[j], iq = idxq[j], iv = idxv[j];
       // configurations a -> b of the pair: (x_t, x_{t+1}) or (xref_t, x_t)
       const bool ref = pi >= T - 1;
       const int t = ref ? pi - (T - 1) : pi;
@@ -353,24 +381,31 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
       auto qa = [&](int k) -> double { return ref ? (double)qrp[k] : qap[k]; };
       auto qb = [&](int k) -> double { return qbp[k]; };
       double* out = (ref ? dr : dd) + t * nv;
-      if (jt == BR_JOINT_FREE_FLYER) {
-        const DPose a{d3(qa(0), qa(1), qa(2)), make_double4(qa(3), qa(4), qa(5), qa(6))};
-        const DPose b{d3(qb(0), qb(1), qb(2)), make_double4(qb(3), qb(4), qb(5), qb(6))};
+      if (jt == BR_JOINT_FREE_FLYER || jt == BR_JOINT_SPHERICAL) {  // one log site
+        const bool ff = jt == BR_JOINT_FREE_FLYER;
+        const int k = ff ? 3 : 0;
+        const double4 ra = make_double4(qa(k), qa(k + 1), qa(k + 2), qa(k + 3));
+        const double4 rb = make_double4(qb(k), qb(k + 1), qb(k + 2), qb(k + 3));
+        DPose rel{d3(0.0, 0.0, 0.0), dqmul(dqconj(ra), rb)};
+        if (ff) rel.t = dqrot(dqconj(ra), dsub(d3(qb(0), qb(1), qb(2)), d3(qa(0), qa(1), qa(2))));
+        else rel.q = dqnormalize(rel.q);
         double3 v, w;
-        dse3_log(dcompose(dinverse(a), b), v, w);
-        out[iv] = v.x; out[iv + 1] = v.y; out[iv + 2] = v.z;
-        out[iv + 3] = w.x; out[iv + 4] = w.y; out[iv + 5] = w.z;
-      } else if (jt == BR_JOINT_SPHERICAL) {
-        const double3 w = dso3_log(dqnormalize(dqmul(dqconj(make_double4(qa(0), qa(1), qa(2), qa(3))),
-                                                     make_double4(qb(0), qb(1), qb(2), qb(3)))));
-        out[iv] = w.x; out[iv + 1] = w.y; out[iv + 2] = w.z;
-      } else if (jt == BR_JOINT_PLANAR || jt == BR_JOINT_REVOLUTE_UNBOUNDED) {
+        dse3_log(rel, v, w);
+        if (ff) { out[iv] = v.x; out[iv + 1] = v.y; out[iv + 2] = v.z; }
+        const int o = iv + k;
+        out[o] = w.x; out[o + 1] = w.y; out[o + 2] = w.z;
+      } else {                                                    // planar, unbounded revolute
         const int k = jt == BR_JOINT_PLANAR ? 2 : 0;
         if (k) { out[iv] = qb(0) - qa(0); out[iv + 1] = qb(1) - qa(1); }
         out[iv + k] = atan2(qb(k + 1), qb(k)) - atan2(qa(k + 1), qa(k));
-      } else {
-        for (int k = 0; k < nvj; ++k) out[iv + k] = qb(k) - qa(k);
       }
+    }
+    for (int e = tid; e < n; e += NT) {
+      const int t = divv.div(e), iq = dofq[e - t * nv];
+      if (iq < 0) continue;
+      const double v = xs[t * nq + iq];
+      if (t < T - 1) dd[e] = xs[(t + 1) * nq + iq] - v;
+      dr[e] = v - (double)xref[t * nq + iq];
     }
     __syncthreads();
   };
@@ -378,34 +413,35 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
   // (free_flyer.py:47-51), spherical normalize(q . exp(w)) (spherical.py:52-56), unbounded
   // revolute / planar angle atan2(s, c) + v as (cos, sin) (revolute.py:223-231, planar.py:61-68)
   auto retract_knots = [&]() {
-    for (int e = tid; e < T * nj; e += NT) {
-      const int t = divj.div(e), j = e - t * nj;
-      const int jt = jtype[j], nvj = joint_nv(jt);
-      if (nvj == 0) continue;
-      const int iq = idxq[j], iv = idxv[j];
+    const int nh = heavy[0];
+    for (int e = tid; e < T * nh; e += NT) {
+      const int hj = e / T, t = e - hj * T, j = heavy[1 + hj];
+      const int jt = jtype[j], iq = idxq[j], iv = idxv[j];
       const double* q = x + t * nq;
       const double* dv = delta + t * nv;
       double* o = xn + t * nq;
-      if (jt == BR_JOINT_FREE_FLYER) {
-        const DPose a{d3(q[iq], q[iq + 1], q[iq + 2]), make_double4(q[iq + 3], q[iq + 4], q[iq + 5], q[iq + 6])};
-        DPose b = dcompose(a, dse3_exp(d3(dv[iv], dv[iv + 1], dv[iv + 2]), d3(dv[iv + 3], dv[iv + 4], dv[iv + 5])));
+      if (jt == BR_JOINT_FREE_FLYER || jt == BR_JOINT_SPHERICAL) {  // one exp site
+        const bool ff = jt == BR_JOINT_FREE_FLYER;
+        const int k = ff ? 3 : 0;
+        const double3 v = ff ? d3(dv[iv], dv[iv + 1], dv[iv + 2]) : d3(0.0, 0.0, 0.0);
+        const DPose a{ff ? d3(q[iq], q[iq + 1], q[iq + 2]) : d3(0.0, 0.0, 0.0),
+                      make_double4(q[iq + k], q[iq + k + 1], q[iq + k + 2], q[iq + k + 3])};
+        DPose b = dcompose(a, dse3_exp(v, d3(dv[iv + k], dv[iv + k + 1], dv[iv + k + 2])));
         b.q = dqnormalize(b.q);
-        o[iq] = b.t.x; o[iq + 1] = b.t.y; o[iq + 2] = b.t.z;
-        o[iq + 3] = b.q.x; o[iq + 4] = b.q.y; o[iq + 5] = b.q.z; o[iq + 6] = b.q.w;
-      } else if (jt == BR_JOINT_SPHERICAL) {
-        const double4 r = dqnormalize(dqmul(make_double4(q[iq], q[iq + 1], q[iq + 2], q[iq + 3]),
-                                            dse3_exp(d3(0.0, 0.0, 0.0), d3(dv[iv], dv[iv + 1], dv[iv + 2])).q));
-        o[iq] = r.x; o[iq + 1] = r.y; o[iq + 2] = r.z; o[iq + 3] = r.w;
-      } else if (jt == BR_JOINT_PLANAR || jt == BR_JOINT_REVOLUTE_UNBOUNDED) {
+        if (ff) { o[iq] = b.t.x; o[iq + 1] = b.t.y; o[iq + 2] = b.t.z; }
+        o[iq + k] = b.q.x; o[iq + k + 1] = b.q.y; o[iq + k + 2] = b.q.z; o[iq + k + 3] = b.q.w;
+      } else {                                                    // planar, unbounded revolute
         const int k = jt == BR_JOINT_PLANAR ? 2 : 0;
         if (k) { o[iq] = q[iq] + dv[iv]; o[iq + 1] = q[iq + 1] + dv[iv + 1]; }
         double sn, cs;
         sincos(atan2(q[iq + k + 1], q[iq + k]) + dv[iv + k], &sn, &cs);
         o[iq + k] = cs;
         o[iq + k + 1] = sn;
-      } else {
-        for (int k = 0; k < nvj; ++k) o[iq + k] = q[iq + k] + dv[iv + k];
       }
+    }
+    for (int e = tid; e < n; e += NT) {
+      const int t = divv.div(e), iq = dofq[e - t * nv];
+      if (iq >= 0) xn[t * nq + iq] = x[t * nq + iq] + delta[e];
     }
   };
   // total cost 0.5 |r|^2 at xs (pose terms evaluated into rg / rs)
@@ -440,20 +476,9 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
     }
     return 0.5 * (acc + pc);
   };
-  // J^T J of the pose terms (packed lower) and g = J^T r at x; returns |g|
+  // pose Jacobians and g = J^T r at x; returns |g|
   auto build = [&]() -> double {
     pose_terms(x, true, true);                        // FK and xi of x from the cost evaluation of x
-    const int npk = nv * (nv + 1) / 2;
-    for (int e = tid; e < npk; e += NT) {
-      const int2 ab = tri_decode(e);
-      double a = 0.0, b = 0.0;
-      for (int r = 0; r < 6; ++r) {
-        if (has_goal) a += Jg[r * nv + ab.x] * Jg[r * nv + ab.y];
-        if (has_start) b += Js[r * nv + ab.x] * Js[r * nv + ab.y];
-      }
-      jtjg[e] = wg * wg * a;
-      jtjs[e] = ws * ws * b;
-    }
     double gg = 0.0;
     for (int e = tid; e < n; e += NT) {
       const int t = divv.div(e), i = e - t * nv;
@@ -510,32 +535,119 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
   // interior columns of the boundary knots: h0 = H[(t, i), (0, i)], hT = H[(t, i), (T-1, i)]
   auto h0_at = [&](int t) -> double { return t == 1 ? hoff1(0) : (t == 2 ? c2 : 0.0); };
   auto hT_at = [&](int t) -> double { return t == T - 2 ? hoff1(T - 2) : (t == T - 3 ? c2 : 0.0); };
-  // solve (J^T J + damp I) delta = -g; false when a pivot is not positive.
-  // Interior knots 1..T-2 of DOF i form the pentadiagonal P_i = L D L^T (thread i).  With
-  // z = L^-1 v, the Schur complement terms are h^T P_i^-1 k = sum_p z_h[p] z_k[p] / D[p], so
-  // one forward pass gives S = H_bb - H_bI P^-1 H_Ib and rb = -g_b - H_bI P^-1 (-g_I) without
-  // storing P^-1 h0 and P^-1 hT; after the boundary solve, the interior step is one more
-  // banded solve with right-hand side -g_I - h0 delta_0 - hT delta_{T-1}.
-  // Twisted factorization (m = T - 2 >= kTwistMin interior knots): the band of DOF i is
-  // factored from both ends at once, thread 2i taking rows 0..k-1 top-down (L D L^T) and
-  // thread 2i + 1 rows m-1..k+2 bottom-up (U E U^T), k = m / 2, which halves the dependent
-  // chain; both then reduce the 2 x 2 block of rows k, k+1 from the two sides' updates.  The
-  // multipliers of the rows into the middle block are kept in the free slots of rows k, k+1
-  // (bl1), every second-neighbour multiplier is c2 times a stored reciprocal pivot.  With
-  // z = M^-1 v the twisted forward substitution, h^T P^-1 v is the sum over the top and bottom
-  // rows of z_h z_v / pivot plus the middle block's r_h^T B^-1 r_v.
-  constexpr int kTwistMin = 8;
-  auto newton_solve = [&](double damp) -> bool {
-    const int m = T - 2;
-    const bool tw = m >= kTwistMin;
+  // solve (J^T J + damp I) delta = -g; false when a pivot is not positive.  Interior knots 1..T-2 of
+  // DOF i form the pentadiagonal P_i, with y = -g_I and the columns h0, hT that tie it to knots 0 and
+  // T-1.  The boundary system is S = H_bb - H_bI P^-1 H_Ib with right-hand side -g_b - H_bI P^-1 y; its
+  // inner products h^T P^-1 k are sums of z_h z_k / pivot over the elimination (z = L^-1 v).
+  const int m = T - 2;
+  const double h1 = -4.0 * c2;                        // H[(p+1), (p)] inside the interior
+
+  // Twisted elimination, two threads per DOF (for more DOFs than cyclic reduction has warps): thread 2i
+  // takes rows 0..k-1 top-down (L D L^T), thread 2i + 1 rows m-1..k+2 bottom-up, k = m / 2, and both then
+  // reduce the 2 x 2 block of rows k, k+1 from the two sides' updates.  The multipliers into the middle
+  // block are kept in the free slots of rows k, k+1 (bl1), every second-neighbour multiplier is c2 times
+  // a stored reciprocal pivot.  h0 is zero in the bottom rows and hT in the top rows, so a side carries
+  // y and one column.  The diagonal waits in the slots of the reciprocals that replace it (bdi), written
+  // by the whole block: its limit tests are not on the chain of pivots.
+  const unsigned tmask = __ballot_sync(0xffffffffu, tid < 2 * nv);
+  auto interior_twisted = [&](double damp) __attribute__((always_inline)) -> bool {
     const int km = m / 2;
     bool good = true;
-    double suu = 0.0, suw = 0.0, sww = 0.0, suy = 0.0, swy = 0.0;
-    const double h1 = -4.0 * c2;                    // H[(p+1), (p)] inside the interior
-    if (!tw && tid < nv) {
+    for (int e = tid; e < m * nv; e += NT) {
+      const int p = divv.div(e);
+      bdi[e] = hdiag(p + 1, e - p * nv, damp);
+    }
+    __syncthreads();
+    if (tid < 2 * nv) {
+      const int i = tid >> 1, side = tid & 1;
+      // side 0: p = 0, 1, .., km-1; side 1: p = m-1, m-2, .., km+2 (the same recurrence on
+      // the reversed band: diagonal, off-diagonals h1 and c2 are symmetric)
+      const int p0 = side ? m - 1 : 0, dir = side ? -1 : 1, steps = side ? m - km - 2 : km;
+      const int step = dir * nv;
+      // row q: multiplier l1 = e / d_(q-1) with e = h1 - c2 l1_(q-1), pivot d = hd - e^2 / d_(q-1)
+      // - c2^2 / d_(q-2): from one reciprocal to the next only e^2 / d_(q-1), everything else is ready
+      double di1 = 0.0, di2 = 0.0, e1 = 0.0, svv = 0.0, svy = 0.0;
+      double y1 = 0, y2 = 0, u1 = 0, u2 = 0;
+      int o = p0 * nv + i;
+      double hd = bdi[o], gy = -g[o + nv];
+      double ub = -2.0 * c2, ub_n = c2;             // h0 = (-2, 1, 0, ...) c2 from the top, hT the same from the bottom
+#pragma unroll 4
+      for (int q = 0; q < steps; ++q) {             // a bad pivot runs on: the result is refused below
+        const double hd_n = bdi[o + step], gy_n = -g[o + step + nv];  // the next row's (a middle row's after the last)
+        const double l2 = c2 * di2;
+        const double dp = (hd - c2 * l2) - e1 * e1 * di1;
+        good = good && dp > 0.0;
+        const double dip = fast_rcp(dp);
+        const double l1 = e1 * di1;
+        bl1[o] = l1; bdi[o] = dip;
+        const double y = (gy - l2 * y2) - l1 * y1;
+        const double u = (ub - l2 * u2) - l1 * u1;
+        svv += u * u * dip;
+        svy += u * y * dip;
+        e1 = h1 - c2 * l1;
+        di2 = di1; di1 = dip;
+        y2 = y1; y1 = y; u2 = u1; u1 = u;
+        ub = ub_n; ub_n = 0.0;
+        o += step; hd = hd_n; gy = gy_n;
+      }
+      // this side's multipliers into the middle block: the adjacent middle row (km for the top,
+      // km + 1 for the bottom) from this side's last two rows, the far middle row from its last
+      const double n1 = e1 * di1, n2 = c2 * di2, f1 = c2 * di1;
+      const int near = side ? km + 1 : km;
+      // updates of the middle block: near diagonal, off-diagonal, far diagonal; right-hand sides
+      const double a_near = n1 * e1 + n2 * c2, a_off = c2 * n1, a_far = f1 * c2;
+      const double ry_near = n1 * y1 + n2 * y2, ry_far = f1 * y1;
+      const double ru_near = n1 * u1 + n2 * u2, ru_far = f1 * u1;
+      const double g0 = -g[(km + 1) * nv + i], g1 = -g[(km + 2) * nv + i];
+      const double hd0 = bdi[km * nv + i], hd1 = bdi[(km + 1) * nv + i];
+      // the other side's updates (lanes 2i, 2i + 1 of one warp)
+      const double o_near = __shfl_xor_sync(tmask, a_near, 1), o_off = __shfl_xor_sync(tmask, a_off, 1),
+                   o_far = __shfl_xor_sync(tmask, a_far, 1);
+      const double oy_near = __shfl_xor_sync(tmask, ry_near, 1), oy_far = __shfl_xor_sync(tmask, ry_far, 1);
+      const double ou_near = __shfl_xor_sync(tmask, ru_near, 1), ou_far = __shfl_xor_sync(tmask, ru_far, 1);
+      const double osvv = __shfl_xor_sync(tmask, svv, 1), osvy = __shfl_xor_sync(tmask, svy, 1);
+      good = __shfl_xor_sync(tmask, (int)good, 1) && good;
+      bl1[near * nv + i] = n1;
+      // middle block in (top, bottom) order, the same on both lanes
+      const double B00 = hd0 - (side ? o_near : a_near) - (side ? a_far : o_far);
+      const double B10 = h1 - a_off - o_off;
+      const double B11 = hd1 - (side ? o_far : a_far) - (side ? a_near : o_near);
+      const double ry0 = g0 - (side ? oy_near : ry_near) - (side ? ry_far : oy_far);
+      const double ry1 = g1 - (side ? oy_far : ry_far) - (side ? ry_near : oy_near);
+      // column h0 comes from the top side, hT from the bottom side
+      const double ru0 = -(side ? ou_near : ru_near), ru1 = -(side ? ou_far : ru_far);
+      const double rw0 = -(side ? ru_far : ou_far), rw1 = -(side ? ru_near : ou_near);
+      good = good && B00 > 0.0;
+      const double dk = good ? fast_rcp(B00) : 0.0;
+      const double lm = B10 * dk;
+      const double D1 = B11 - lm * B10;
+      good = good && D1 > 0.0;
+      const double dk1 = good ? fast_rcp(D1) : 0.0;
+      // a^T B^-1 b = a0 b0 / B00 + (a1 - l a0)(b1 - l b0) / D1
+      auto bq = [&](double a0, double a1, double b0, double b1) {
+        return a0 * b0 * dk + (a1 - lm * a0) * (b1 - lm * b0) * dk1;
+      };
+      if (side == 0) {
+        bdi[km * nv + i] = dk; bdi[(km + 1) * nv + i] = dk1;
+        schur[i] = svv + bq(ru0, ru1, ru0, ru1);
+        schur[nv + i] = bq(ru0, ru1, rw0, rw1);
+        schur[2 * nv + i] = osvv + bq(rw0, rw1, rw0, rw1);
+        schur[3 * nv + i] = svy + bq(ru0, ru1, ry0, ry1);
+        schur[4 * nv + i] = osvy + bq(rw0, rw1, ry0, ry1);
+      }
+    }
+    return good;
+  };
+
+  // Few interior knots: thread i runs DOF i's band from the top.
+  constexpr int kTwistMin = 8;
+  auto interior_plain = [&](double damp) __attribute__((always_inline)) -> bool {
+    bool good = true;
+    if (tid < nv) {
       const int i = tid;
       double d1 = 0.0, di1 = 0.0, di2 = 0.0, l1p = 0.0;
       double y1 = 0, y2 = 0, u1 = 0, u2 = 0, w1 = 0, w2 = 0;
+      double suu = 0.0, suw = 0.0, sww = 0.0, suy = 0.0, swy = 0.0;
       for (int p = 0; p < m; ++p) {
         const int t = p + 1;
         const double l2 = (p >= 2) ? c2 * di2 : 0.0;
@@ -552,212 +664,239 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
         di2 = di1; di1 = dip; d1 = dp; l1p = l1;
         y2 = y1; y1 = y; u2 = u1; u1 = u; w2 = w1; w1 = w;
       }
+      schur[i] = suu; schur[nv + i] = suw; schur[2 * nv + i] = sww; schur[3 * nv + i] = suy; schur[4 * nv + i] = swy;
     }
-    const unsigned tmask = __ballot_sync(0xffffffffu, tid < 2 * nv);
-    if (tw && tid < 2 * nv) {
-      const int i = tid >> 1, side = tid & 1;
-      // side 0: p = 0, 1, .., km-1; side 1: p = m-1, m-2, .., km+2 (the same recurrence on
-      // the reversed band: diagonal, off-diagonals h1 and c2 are symmetric)
-      const int p0 = side ? m - 1 : 0, dir = side ? -1 : 1, steps = side ? m - km - 2 : km;
-      double d1 = 0.0, di1 = 0.0, di2 = 0.0, l1p = 0.0;
-      double y1 = 0, y2 = 0, u1 = 0, u2 = 0, w1 = 0, w2 = 0;
-      for (int q = 0; q < steps; ++q) {
-        const int p = p0 + dir * q, t = p + 1;
-        const double l2 = (q >= 2) ? c2 * di2 : 0.0;
-        const double l1 = (q >= 1) ? (h1 - c2 * l1p) * di1 : 0.0;
-        const double dp = hdiag(t, i, damp) - l1 * l1 * d1 - l2 * c2;
-        if (!(dp > 0.0)) { good = false; break; }
-        const double dip = fast_rcp(dp);
-        bl1[p * nv + i] = l1; bdi[p * nv + i] = dip;
-        const double y = -g[t * nv + i] - l1 * y1 - l2 * y2;
-        const double u = h0_at(t) - l1 * u1 - l2 * u2;
-        const double w = hT_at(t) - l1 * w1 - l2 * w2;
-        suu += u * u * dip; suw += u * w * dip; sww += w * w * dip;
-        suy += u * y * dip; swy += w * y * dip;
-        di2 = di1; di1 = dip; d1 = dp; l1p = l1;
-        y2 = y1; y1 = y; u2 = u1; u1 = u; w2 = w1; w1 = w;
-      }
-      // this side's multipliers into the middle block: the adjacent middle row (km for the top,
-      // km + 1 for the bottom) from this side's last two rows, the far middle row from its last
-      const double n1 = (h1 - c2 * l1p) * di1, n2 = c2 * di2, f1 = c2 * di1;
-      const int near = side ? km + 1 : km;
-      bl1[near * nv + i] = n1;
-      // updates of the middle block: near diagonal, off-diagonal, far diagonal; right-hand sides
-      const double a_near = n1 * n1 * d1 + n2 * c2, a_off = c2 * n1, a_far = f1 * c2;
-      const double ry_near = n1 * y1 + n2 * y2, ry_far = f1 * y1;
-      const double ru_near = n1 * u1 + n2 * u2, ru_far = f1 * u1;
-      const double rw_near = n1 * w1 + n2 * w2, rw_far = f1 * w1;
-      // the other side's updates (lanes 2i, 2i + 1 of one warp)
-      const double o_near = __shfl_xor_sync(tmask, a_near, 1), o_off = __shfl_xor_sync(tmask, a_off, 1),
-                   o_far = __shfl_xor_sync(tmask, a_far, 1);
-      const double oy_near = __shfl_xor_sync(tmask, ry_near, 1), oy_far = __shfl_xor_sync(tmask, ry_far, 1);
-      const double ou_near = __shfl_xor_sync(tmask, ru_near, 1), ou_far = __shfl_xor_sync(tmask, ru_far, 1);
-      const double ow_near = __shfl_xor_sync(tmask, rw_near, 1), ow_far = __shfl_xor_sync(tmask, rw_far, 1);
-      const double osuu = __shfl_xor_sync(tmask, suu, 1), osuw = __shfl_xor_sync(tmask, suw, 1),
-                   osww = __shfl_xor_sync(tmask, sww, 1), osuy = __shfl_xor_sync(tmask, suy, 1),
-                   oswy = __shfl_xor_sync(tmask, swy, 1);
-      good = good && __shfl_xor_sync(tmask, (int)good, 1);
-      // middle block in (top, bottom) order, the same on both lanes
-      const double tA = side ? o_near : a_near, tF = side ? o_far : a_far, tO = side ? o_off : a_off;
-      const double bA = side ? a_near : o_near, bF = side ? a_far : o_far, bO = side ? a_off : o_off;
-      const int t0 = km + 1, t1 = km + 2;
-      const double B00 = hdiag(t0, i, damp) - tA - bF;
-      const double B10 = h1 - tO - bO;
-      const double B11 = hdiag(t1, i, damp) - tF - bA;
-      auto mid = [&](double v0, double v1, double top_near, double top_far, double bot_near, double bot_far,
-                     double& r0, double& r1) {
-        r0 = v0 - top_near - bot_far;
-        r1 = v1 - top_far - bot_near;
-      };
-      double ry0, ry1, ru0, ru1, rw0, rw1;
-      mid(-g[t0 * nv + i], -g[t1 * nv + i], side ? oy_near : ry_near, side ? oy_far : ry_far,
-          side ? ry_near : oy_near, side ? ry_far : oy_far, ry0, ry1);
-      mid(h0_at(t0), h0_at(t1), side ? ou_near : ru_near, side ? ou_far : ru_far,
-          side ? ru_near : ou_near, side ? ru_far : ou_far, ru0, ru1);
-      mid(hT_at(t0), hT_at(t1), side ? ow_near : rw_near, side ? ow_far : rw_far,
-          side ? rw_near : ow_near, side ? rw_far : ow_far, rw0, rw1);
-      good = good && B00 > 0.0;
-      const double dk = good ? fast_rcp(B00) : 0.0;
-      const double lm = B10 * dk;
-      const double D1 = B11 - lm * B10;
-      good = good && D1 > 0.0;
-      const double dk1 = good ? fast_rcp(D1) : 0.0;
-      if (side == 0) { bdi[km * nv + i] = dk; bdi[(km + 1) * nv + i] = dk1; }
-      // a^T B^-1 b = a0 b0 / B00 + (a1 - l a0)(b1 - l b0) / D1
-      auto bq = [&](double a0, double a1, double b0, double b1) {
-        return a0 * b0 * dk + (a1 - lm * a0) * (b1 - lm * b0) * dk1;
-      };
-      suu += osuu + bq(ru0, ru1, ru0, ru1);
-      suw += osuw + bq(ru0, ru1, rw0, rw1);
-      sww += osww + bq(rw0, rw1, rw0, rw1);
-      suy += osuy + bq(ru0, ru1, ry0, ry1);
-      swy += oswy + bq(rw0, rw1, ry0, ry1);
-    }
+    return good;
+  };
+
+  const bool tw = m >= kTwistMin;
+
+  auto newton_solve = [&](double damp) __attribute__((always_inline)) -> bool {
+    for (int b = tid; b < nb; b += NT) sd[b] = hdiag(b < nv ? 0 : T - 1, b < nv ? b : b - nv, damp);
+    const bool good = tw ? interior_twisted(damp) : interior_plain(damp);
     if (__syncthreads_or(!good)) return false;
-    // boundary block H_bb, packed lower: b = i for (knot 0, DOF i), nv + i for (knot T-1, DOF i)
-    const int nbp = nb * (nb + 1) / 2;
-    for (int e = tid; e < nbp; e += NT) {
-      const int2 rc = tri_decode(e);
-      const int r = rc.x, cc = rc.y;
-      const int kr = r >= nv, kc = cc >= nv, ir = r - kr * nv, ic = cc - kc * nv;
-      double h = 0.0;
-      if (kr == kc) {
-        const int pe = ir >= ic ? tri_at(ir, ic) : tri_at(ic, ir);
-        if (kr == 0 && has_start) h = jtjs[pe];
-        if (kr == 1 && has_goal) h = jtjg[pe];
-        if (ir == ic) h += hdiag(kr ? T - 1 : 0, ir, damp);
-      } else if (ir == ic && T == 3) {
-        h = c2;                                                    // row 0 couples knots 0 and 2
-      }
-      Sb[e] = h;
-    }
-    __syncthreads();
-    if (tw ? (tid < 2 * nv && (tid & 1) == 0) : tid < nv) {
-      const int i = tw ? tid >> 1 : tid;
-      Sb[tri_at(i, i)] -= suu;
-      Sb[tri_at(nv + i, i)] -= suw;
-      Sb[tri_at(nv + i, nv + i)] -= sww;
-      rb[i] = -g[i] - suy;
-      rb[nv + i] = -g[(T - 1) * nv + i] - swy;
-    }
-    __syncthreads();
-    for (int k = 0; k < nb; ++k) {                                  // chol(S), lower, in place
-      const double dkk = Sb[tri_at(k, k)];
-      if (!(dkk > 0.0)) return false;                               // every thread read the same value
-      const double inv = fast_rsqrt(dkk);
-      __syncthreads();
-      for (int r = k + 1 + tid; r < nb; r += NT) Sb[tri_at(r, k)] *= inv;
-      if (tid == 0) { Sb[tri_at(k, k)] = dkk * inv; sdi[k] = inv; }
-      __syncthreads();
-      // trailing update S[r][cc] -= L[r][k] L[cc][k], k < cc <= r < nb, as packed pairs
-      const int np = (nb - k - 1) * (nb - k) / 2;
-      for (int pp = tid; pp < np; pp += NT) {
-        const int2 ab = tri_decode(pp);
-        const int r = ab.x + k + 1, cc = ab.y + k + 1;
-        Sb[tri_at(r, cc)] -= Sb[tri_at(r, k)] * Sb[tri_at(cc, k)];
-      }
-      __syncthreads();
-    }
-    // z = S^-1 rb
-    if (nb <= kWarp) {
-      if (warp == 0) {                      // lane b owns entry b; one finished entry broadcast per step
-        double v = (lane < nb) ? rb[lane] : 0.0;
-        for (int j = 0; j < nb; ++j) {
-          const double zj = __shfl_sync(0xffffffffu, v, j) * sdi[j];
-          if (lane == j) v = zj;
-          else if (lane > j && lane < nb) v -= Sb[tri_at(lane, j)] * zj;
+    // boundary system, packed lower: b = i for (knot 0, DOF i), nv + i for (knot T-1, DOF i); its
+    // right-hand side is row nb, so that the factorization also substitutes forward
+    for (int kb = 0; kb < 2; ++kb) {                   // the two dense blocks, four rows of a warp at once
+      const double* J = kb ? Jg : Js;
+      const double wj = kb ? (has_goal ? wg * wg : 0.0) : (has_start ? ws * ws : 0.0);
+      for (int r0 = 4 * warp; r0 < nv; r0 += 4 * NW)
+        for (int ic = lane; ic < nv && ic < r0 + 4; ic += kWarp) {
+          double h[4] = {0.0, 0.0, 0.0, 0.0};
+          if (wj > 0.0) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+              const double jc = J[k * nv + ic] * wj;
+#pragma unroll
+              for (int q = 0; q < 4; ++q) h[q] += J[k * nv + (r0 + q < nv ? r0 + q : r0)] * jc;
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int ir = r0 + q;
+            if (ir >= nv || ic > ir) continue;
+            if (ir == ic) h[q] += sd[kb * nv + ir] - schur[2 * kb * nv + ir];
+            Sb[tri_at(kb * nv + ir, kb * nv + ic)] = h[q];
+          }
         }
-        for (int j = nb - 1; j >= 0; --j) {
-          const double zj = __shfl_sync(0xffffffffu, v, j) * sdi[j];
-          if (lane == j) v = zj;
-          else if (lane < j) v -= Sb[tri_at(j, lane)] * zj;
-        }
-        if (lane < nb) zb[lane] = v;
-      }
-    } else {                                // column-oriented substitutions over the block
-      for (int j = 0; j < nb; ++j) {        // L y = rb (rb overwritten by the partial sums)
-        const double yj = rb[j] * sdi[j];
-        for (int r = j + 1 + tid; r < nb; r += NT) rb[r] -= Sb[tri_at(r, j)] * yj;
-        if (tid == 0) zb[j] = yj;
-        __syncthreads();
-      }
-      for (int j = nb - 1; j >= 0; --j) {   // L^T z = y (zb overwritten in place)
-        const double zj = zb[j] * sdi[j];
-        __syncthreads();
-        for (int r = tid; r < j; r += NT) zb[r] -= Sb[tri_at(j, r)] * zj;
-        if (tid == 0) zb[j] = zj;
-        __syncthreads();
-      }
+    }
+    for (int r = warp; r < nv; r += NW)                // knots 0 and T-1 meet on each DOF's own band only
+      for (int ic = lane; ic < nv; ic += kWarp)        // (T = 3: acceleration row 0 couples them)
+        Sb[tri_at(nv + r, ic)] = ic == r ? (T == 3 ? c2 : 0.0) - schur[nv + r] : 0.0;
+    for (int cc = tid; cc < nb; cc += NT) {
+      const int kc = cc >= nv, ic = cc - kc * nv;
+      Sb[tri_at(nb, cc)] = -g[(kc ? T - 1 : 0) * nv + ic] - schur[(3 + kc) * nv + ic];
     }
     __syncthreads();
-    // interior step of DOF i: P_i d = -g_I - h0 z(knot 0) - hT z(knot T-1); forward into delta,
-    // then backward in place (twisted: from both ends to the middle block and back out)
+    // L D L^T of S in panels of kPan columns: warp 0 eliminates the panel on its first 32 rows (lane r row
+    // k0 + r; every lane carries the pivots, so that one reciprocal and one multiply-add separate two of
+    // them), one thread per row the rows below, and the block updates the rest of S: one entry per thread
+    // while they are few, else 4 x 4 tiles.  The panel's entries stay as L; sdi 1 / pivot, sd pivot.
+    constexpr int kPan = 8;
+    bool pos = true;
+    for (int k0 = 0; k0 < nb; k0 += kPan) {
+      const int pw = nb - k0 < kPan ? nb - k0 : kPan, k1 = k0 + pw;
+      if (warp == 0) {
+        const int r = k0 + lane < nb ? k0 + lane : nb;
+        double* row = Sb + tri_at(r, k0);
+        double a[kPan], myd = 1.0, myi = 1.0;
+#pragma unroll
+        for (int j = 0; j < kPan; ++j) a[j] = j < pw && k0 + j <= r ? row[j] : 0.0;
+        double d = __shfl_sync(0xffffffffu, a[0], 0);
+#pragma unroll
+        for (int j = 0; j < kPan; ++j) {
+          if (j >= pw) break;
+          pos = pos && d > 0.0;
+          const double aj = a[j];
+          double bj[kPan];
+#pragma unroll
+          for (int k = j + 1; k < kPan; ++k) bj[k] = __shfl_sync(0xffffffffu, aj, k);
+          const double nd = j + 1 < kPan ? __shfl_sync(0xffffffffu, a[j + 1 < kPan ? j + 1 : 0], j + 1) : 1.0;
+          const double b1 = j + 1 < kPan ? bj[j + 1 < kPan ? j + 1 : 0] : 0.0, bb = b1 * b1;
+          const double ri = fast_rcp(d);
+          const double lj = aj * ri;
+#pragma unroll
+          for (int k = j + 1; k < kPan; ++k) a[k] -= lj * bj[k];
+          a[j] = lj;
+          myd = lane == j ? d : myd;
+          myi = lane == j ? ri : myi;
+          d = nd - bb * ri;
+        }
+        if (lane < pw) { sd[k0 + lane] = myd; sdi[k0 + lane] = myi; }
+        if (k0 + lane <= nb) {
+#pragma unroll
+          for (int j = 0; j < kPan; ++j)
+            if (j < pw && j < lane) row[j] = a[j];
+        }
+      }
+      if (__syncthreads_or(warp == 0 && !pos)) return false;
+      if (k0 + kWarp <= nb) {
+        for (int r = k0 + kWarp + tid; r <= nb; r += NT) {           // W L^T = S, stored as W / pivot
+          double w[kPan];
+          double* row = Sb + tri_at(r, k0);
+#pragma unroll
+          for (int j = 0; j < kPan; ++j) w[j] = j < pw ? row[j] : 0.0;
+#pragma unroll
+          for (int j = 0; j < kPan; ++j) {
+            if (j < pw) {
+#pragma unroll
+              for (int k = j + 1; k < kPan; ++k)
+                if (k < pw) w[k] -= w[j] * Sb[tri_at(k0 + k, k0 + j)];
+              row[j] = w[j] * sdi[k0 + j];
+            }
+          }
+        }
+        __syncthreads();
+      }
+      if (k1 >= nb) break;
+      // S[r][c] -= sum_j L[r][j] pivot_j L[c][j] for k1 <= c <= r <= nb, c < nb (a full panel here)
+      const int nr = nb + 1 - k1, ne = nr * (nr + 1) / 2 - 1;
+      if (ne <= 4 * NT) {
+        for (int e = tid; e < ne; e += NT) {
+          const int2 rc = tri_decode(e);
+          const double *lr = Sb + tri_at(k1 + rc.x, k0), *lc = Sb + tri_at(k1 + rc.y, k0);
+          double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+          for (int j = 0; j < kPan; j += 2) {
+            s0 += lr[j] * (lc[j] * sd[k0 + j]);
+            s1 += lr[j + 1] * (lc[j + 1] * sd[k0 + j + 1]);
+          }
+          Sb[tri_at(k1 + rc.x, k1 + rc.y)] -= s0 + s1;
+        }
+      } else {
+        const int nt = (nr + 3) >> 2;
+        for (int e = tid; e < nt * (nt + 1) / 2; e += NT) {
+          const int2 ij = tri_decode(e);
+          const int r0 = k1 + 4 * ij.x, c0 = k1 + 4 * ij.y;
+          double acc[4][4];
+          const double *lr[4], *lc[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {                            // rows past the last repeat it (not stored)
+            lr[q] = Sb + tri_at(r0 + q < nb ? r0 + q : nb, k0);
+            lc[q] = Sb + tri_at(c0 + q < nb ? c0 + q : nb, k0);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[q][v] = 0.0;
+          }
+#pragma unroll 4
+          for (int j = 0; j < kPan; ++j) {
+            const double dj = sd[k0 + j];
+            double x[4], y[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { x[q] = lr[q][j]; y[q] = lc[q][j] * dj; }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+              for (int v = 0; v < 4; ++v) acc[q][v] += x[q] * y[v];
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int r = r0 + q, cc = c0 + v;
+              if (r <= nb && cc <= r && cc < nb) Sb[tri_at(r, cc)] -= acc[q][v];
+            }
+        }
+      }
+      __syncthreads();
+    }
+    __syncthreads();
+    // row nb now holds D^-1 L^-1 b: z = L^-T of it, panel by panel from the last
+    for (int e = tid; e < nb; e += NT) zb[e] = Sb[tri_at(nb, e)];
+    __syncthreads();
+    for (int k0 = (nb - 1) / kPan * kPan; k0 >= 0; k0 -= kPan) {
+      const int pw = nb - k0 < kPan ? nb - k0 : kPan;
+      if (warp == 0) {
+        double v = lane < pw ? zb[k0 + lane] : 0.0, lc[kPan];
+#pragma unroll
+        for (int j = 1; j < kPan; ++j) lc[j] = j < pw && lane < j ? Sb[tri_at(k0 + j, k0 + lane)] : 0.0;
+#pragma unroll
+        for (int j = kPan - 1; j >= 1; --j) {
+          const double zj = __shfl_sync(0xffffffffu, v, j);
+          v -= lc[j] * zj;
+        }
+        if (lane < pw) zb[k0 + lane] = v;
+      }
+      __syncthreads();
+      for (int cc = tid; cc < k0; cc += NT) {
+        double v = zb[cc];
+        for (int j = 0; j < pw; ++j) v -= Sb[tri_at(k0 + j, cc)] * zb[k0 + j];
+        zb[cc] = v;
+      }
+      __syncthreads();
+    }
+    // interior step of DOF i: P_i d = y - h0 z(knot 0) - hT z(knot T-1)
     if (tw && tid < 2 * nv) {
+      // forward into delta, then backward in place: from both ends to the middle block and back out
+      const int km = m / 2;
       const int i = tid >> 1, side = tid & 1;
-      const double z0 = zb[i], zT = zb[nv + i];
+      const double z0 = zb[i], zT = zb[nv + i], zs = side ? zT : z0;
       if (side == 0) {
         delta[i] = z0;
         delta[(T - 1) * nv + i] = zT;
       }
-      auto rhs = [&](int t) { return -g[t * nv + i] - h0_at(t) * z0 - hT_at(t) * zT; };
       const int p0 = side ? m - 1 : 0, dir = side ? -1 : 1, steps = side ? m - km - 2 : km;
-      double y1 = 0, y2 = 0;
+      const int step = dir * nv;
+      double y1 = 0, y2 = 0, di2 = 0.0, di1 = 0.0;
+      int o = p0 * nv + i;
+      double l1 = bl1[o], di = bdi[o], gy = -g[o + nv];
       for (int q = 0; q < steps; ++q) {
-        const int p = p0 + dir * q, t = p + 1;
-        const double l1 = bl1[p * nv + i], l2 = (q >= 2) ? c2 * bdi[(p - 2 * dir) * nv + i] : 0.0;
-        const double y = rhs(t) - l1 * y1 - l2 * y2;
-        delta[t * nv + i] = y;
-        y2 = y1; y1 = y;
+        const double l1_n = bl1[o + step], di_n = bdi[o + step], gy_n = -g[o + step + nv];
+        const double rhs = q == 0 ? gy + 2.0 * c2 * zs : q == 1 ? gy - c2 * zs : gy;
+        const double y = (rhs - c2 * di2 * y2) - l1 * y1;
+        delta[o + nv] = y;
+        y2 = y1; y1 = y; di2 = di1; di1 = di;
+        o += step; l1 = l1_n; di = di_n; gy = gy_n;
       }
       // middle block: this side's last two rows, multipliers as in the factorization
-      const int pl = p0 + dir * (steps - 1);                      // this side's last row
       const double n1 = bl1[(side ? km + 1 : km) * nv + i];
-      const double n2 = c2 * bdi[(pl - dir) * nv + i], f1 = c2 * bdi[pl * nv + i];
+      const double n2 = c2 * di2, f1 = c2 * di1;
       const double r_near = n1 * y1 + n2 * y2, r_far = f1 * y1;
       const double o_near = __shfl_xor_sync(tmask, r_near, 1), o_far = __shfl_xor_sync(tmask, r_far, 1);
       const double on1 = __shfl_xor_sync(tmask, n1, 1);
-      const double tn = side ? o_near : r_near, tf = side ? o_far : r_far;
-      const double bn = side ? r_near : o_near, bfar = side ? r_far : o_far;
-      const double r0 = rhs(km + 1) - tn - bfar, r1 = rhs(km + 2) - tf - bn;
+      const double x0r = -g[(km + 1) * nv + i] - (side ? o_near : r_near) - (side ? r_far : o_far);
+      const double x1r = -g[(km + 2) * nv + i] - (side ? o_far : r_far) - (side ? r_near : o_near);
       const double dk = bdi[km * nv + i], dk1 = bdi[(km + 1) * nv + i];
       const double lm = (h1 - c2 * n1 - c2 * on1) * dk;           // B10 / B00 (symmetric in the sides)
-      const double x1 = (r1 - lm * r0) * dk1, x0 = r0 * dk - lm * x1;
+      const double x1 = (x1r - lm * x0r) * dk1, x0 = x0r * dk - lm * x1;
       if (side == 0) {
         delta[(km + 1) * nv + i] = x0;
         delta[(km + 2) * nv + i] = x1;
       }
       // back substitution outwards: x_p = z_p / pivot_p - (near multiplier) x_(p+dir') - c2 / pivot_p x_(p+2dir')
       double xa = side ? x1 : x0, xb = side ? x0 : x1;            // the next two rows towards the middle
+      double ln = n1;                                             // the row towards the middle, relative to p
+      o -= step;
+      double dp = bdi[o], yp = delta[o + nv], lp = bl1[o];
       for (int q = steps - 1; q >= 0; --q) {
-        const int p = p0 + dir * q;
-        const double di = bdi[p * nv + i];
-        const double ln = bl1[(p + dir) * nv + i];                 // the row towards the middle, relative to p
-        const double y = delta[(p + 1) * nv + i] * di - ln * xa - c2 * di * xb;
-        delta[(p + 1) * nv + i] = y;
+        const int on = q > 0 ? o - step : o;
+        const double dp_n = bdi[on], yp_n = delta[on + nv], lp_n = bl1[on];
+        const double y = (yp * dp - c2 * dp * xb) - ln * xa;
+        delta[o + nv] = y;
         xb = xa; xa = y;
+        ln = lp;
+        o = on; dp = dp_n; yp = yp_n; lp = lp_n;
       }
-    }
-    if (!tw && tid < nv) {
+    } else if (!tw && tid < nv) {
       const int i = tid;
       const double z0 = zb[i], zT = zb[nv + i];
       delta[i] = z0;
@@ -785,25 +924,53 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
   };
 
   // ---- GN / LM loop (gauss_newton.py:27-76, levenberg_marquardt.py:83-135) ----
+  // cost_of and newton_solve have ONE call site each (they are inlined: a second one would be a second
+  // copy of the code): the first pass evaluates the start, every later one a trial point, and a last
+  // pass the returned x when the goal gradient is wanted and the final trial was rejected.
   const bool lm = S.optimizer == BR_OPT_LM;
-  double cost = cost_of(x);
-  double lam = lm ? (double)S.lam0 : 0.0;
-  double gnorm = 0.0;
-  bool need = true;
+  const bool want_goal = P.goal_grad && has_goal;
+  double cost = 0.0, lam = lm ? (double)S.lam0 : 0.0, gnorm = 0.0;
+  bool need = true, started = false, at_x = true;
   int status = BR_IK_MAXITER, flags = 0, it = 0;
-  for (; it < S.max_iter; ++it) {
+  const double* xe = x;
+  for (;;) {
+    const double cn = cost_of(xe);
+    if (!started) {
+      started = true;
+      cost = cn;
+    } else if (at_x) {                                             // the last pass
+      break;
+    } else {
+      ++it;
+      if (!isfinite(cn)) flags |= BR_IK_FLAG_NONFINITE;
+      if (!lm || cn < cost) {
+        double* t = x; x = xn; xn = t;
+        at_x = true;
+        cost = cn;
+        need = true;
+        if (lm) lam = fmax(lam / S.factor, (double)S.lam_min);
+        if (gnorm < S.tol) { status = BR_IK_CONVERGED; break; }
+      } else {
+        lam = fmin(lam * S.factor, (double)S.lam_max);
+      }
+    }
+    if (it >= S.max_iter) {
+      if (!want_goal || at_x) break;
+      at_x = true;
+      xe = x;
+      continue;
+    }
     if (need) { gnorm = build(); need = false; }
-    if (!newton_solve(lm ? lam : (double)S.gn_eps)) {
-      flags |= BR_IK_FLAG_REGULARIZED;
-      bool ok = false;
-      double extra = 1e-9;
-      for (int k = 0; k < 8 && !ok; ++k, extra *= 10.0) {
-        ok = newton_solve((lm ? lam : (double)S.gn_eps) + extra);
-      }
-      if (!ok) {
-        for (int e = tid; e < n; e += NT) delta[e] = 0.0;
-        __syncthreads();
-      }
+    bool ok = false;
+    double extra = 0.0;
+    for (int k = 0; k < 9 && !ok; ++k) {                           // retries with diagonal regularisation
+      ok = newton_solve((lm ? lam : (double)S.gn_eps) + extra);
+      if (!ok) flags |= BR_IK_FLAG_REGULARIZED;
+      extra = k == 0 ? 1e-9 : extra * 10.0;
+    }
+    if (!ok) {
+      for (int e = tid; e < n; e += NT) delta[e] = 0.0;
+      __syncthreads();
     }
     if (kManifold) {                                               // Model.integrate per knot (trajopt.py:159-169)
       retract_knots();
@@ -811,29 +978,17 @@ __global__ void __launch_bounds__(kTrajThreads) traj_gn_kernel(const TrajParams 
       for (int e = tid; e < n; e += NT) xn[e] = x[e] + delta[e];
     }
     __syncthreads();
-    const double cn = cost_of(xn);
-    if (!isfinite(cn)) flags |= BR_IK_FLAG_NONFINITE;
-    bool accept = !lm || cn < cost;
-    if (accept) {
-      for (int e = tid; e < nqT; e += NT) x[e] = xn[e];
-      __syncthreads();
-      cost = cn;
-      need = true;
-      if (lm) lam = fmax(lam / S.factor, (double)S.lam_min);
-      if (gnorm < S.tol) { status = BR_IK_CONVERGED; ++it; break; }
-    } else {
-      lam = fmin(lam * S.factor, (double)S.lam_max);
-    }
+    at_x = false;
+    xe = xn;
   }
+  __syncthreads();
   float* xo = P.x + traj * (int64_t)nqT;
   for (int e = tid; e < nqT; e += NT) xo[e] = (float)x[e];
-  if (P.goal_grad && has_goal) {
-    pose_terms(x, false, false);
-    __syncthreads();
+  if (want_goal) {                                                 // rg holds the pose error of x
     if (tid == 0) {
       const double3 v = d3(rg[0], rg[1], rg[2]);
       const double3 w = d3(rg[3], rg[4], rg[5]);
-      const DJrInv Jl = djr_inv_se3<20>(dscale(v, -1.0), dscale(w, -1.0));   // Jl^-1(xi) = Jr^-1(-xi)
+      const DJrInv Jl = djr_inv_se3_rolled<20>(dscale(v, -1.0), dscale(w, -1.0));   // Jl^-1(xi) = Jr^-1(-xi)
       double3 gl, ga;
       djr_inv_T_apply(Jl, v, w, gl, ga);
       const double k = -wg * wg;
@@ -885,15 +1040,17 @@ extern "C" int br_trajopt_solve(const br_tree_t* tree, int32_t frame_id, int64_t
   const size_t bytes = (size_t)L.total * sizeof(double);
   const DeviceInfo& dev = device_info();
   if ((int64_t)bytes > dev.max_smem_optin) return BR_ETOOBIG;
-  auto kern = floating ? traj_gn_kernel<true> : traj_gn_kernel<false>;
-  static int configured[2][16] = {{0}};
-  int& conf = configured[floating ? 1 : 0][dev.device & 15];
+  if (n_traj > 0x7fffffff) return BR_ETOOBIG;
+  const bool wide = n_traj <= dev.sms || 2 * ((int64_t)bytes + 1024) > dev.smem_per_sm;
+  auto kern = floating ? (wide ? traj_gn_kernel<true, 256> : traj_gn_kernel<true, 128>)
+                       : (wide ? traj_gn_kernel<false, 256> : traj_gn_kernel<false, 128>);
+  static int configured[4][16] = {{0}};
+  int& conf = configured[(floating ? 2 : 0) + (wide ? 1 : 0)][dev.device & 15];
   if ((int)bytes > conf) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return (int)e;
     conf = (int)bytes;
   }
-  if (n_traj > 0x7fffffff) return BR_ETOOBIG;
-  kern<<<(unsigned)n_traj, kTrajThreads, bytes, (cudaStream_t)stream>>>(p);
+  kern<<<(unsigned)n_traj, wide ? 256 : 128, bytes, (cudaStream_t)stream>>>(p);
   return (int)cudaGetLastError();
 }
