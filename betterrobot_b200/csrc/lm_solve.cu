@@ -62,7 +62,7 @@ struct LmParams {
 struct TeamLayout {
   int parent, jtype, idxq, idxv, support, cjoint, ckind, caxis, lower, upper;
   int fparent, fplace, tgt, tkind;
-  int dpar, ddep, rowoff, amask, ancd;
+  int ddep, rowoff, ancd;
   int x, xn, qrest, poseA, poseB, ancA, ancB, tw, xi, jri, colw, d, g, delta, jtj, work, misc,
       dinv, sup, nsup;
   int n_ent, anc_stride;  // capacity of the J^T J / factor storage; row length of ancd
@@ -89,19 +89,18 @@ struct TeamLayout {
     jri = take(16 * K * rs); colw = take(8 * nv * rs);
     g = take(nv * rs); delta = take(nv * rs);
     const int ntri = nv * (nv + 1) / 2;
-    n_ent = (ent > 0 && ent < ntri) ? ent : ntri;
+    // one row per DOF: its right-hand side, then its entries, padded to pairs
+    n_ent = ((ent > 0 && ent < ntri) ? ent : ntri) + 2 * nv;
     anc_stride = (dep > 0 && dep < nv) ? dep : (nv > 0 ? nv : 1);
-    jtj = take(n_ent * rs);                    // J^T J, one row per DOF over its ancestors
+    jtj = take(n_ent * rs);                    // -J^T r and J^T J, one row per DOF over its ancestors
     // two targets' J columns (build) / the factor and its right-hand-side slots (solve):
     // in the pose buffer that FK does not return (poseA after an odd number of rounds, else
     // poseB), dead while the normal equations are built and solved, when it is large enough
-    const int wneed = (12 * nv > n_ent + nv ? 12 * nv : n_ent + nv) * rs;
+    const int wneed = (12 * nv > n_ent ? 12 * nv : n_ent) * rs;
     work = wneed <= 14 * nj ? ((rounds & 1) ? poseA : poseB) : take(wneed);
     dinv = take(nv * rs);                      // 1 / L_jj
     ancA = take(nj); ancB = take(nj);
     misc = take(8);
-    amask = take(2 * nv);                      // uint64 strict ancestors of each DOF
-    dpar = take((nv + 3) / 4);                 // int8 parent DOF (-1 at a root)
     ddep = take((nv + 3) / 4);                 // uint8 DOF depth
     rowoff = take((nv + 2) / 2);               // uint16 first entry of each row, nv + 1 values
     ancd = take((nv * anc_stride + 3) / 4);    // uint8 ancestor of DOF c at depth a: ancd[c * anc_stride + a]
@@ -112,9 +111,8 @@ struct TeamLayout {
 };
 
 __device__ __forceinline__ int tri(int i) { return i * (i + 1) / 2; }
-// Largest trunk (root chain above every other DOF) factored in registers by the float64
-// variants: its ntr (ntr + 1) / 2 factor entries and ntr right-hand sides take one lane each
-// of a 32-lane team.
+// Largest trunk (root chain above every other DOF) of a row schedule: its n (n + 1) / 2 factor
+// entries and n right-hand sides take one lane each of a 32-lane team.
 constexpr int kTrunkMax = 6;
 
 
@@ -269,8 +267,6 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
   R* delta = reinterpret_cast<R*>(sm + L.delta);
   R* jtj = reinterpret_cast<R*>(sm + L.jtj);
   R* work = reinterpret_cast<R*>(sm + L.work);
-  unsigned long long* amask = reinterpret_cast<unsigned long long*>(sm + L.amask);
-  signed char* dpar = reinterpret_cast<signed char*>(sm + L.dpar);
   unsigned char* ddep = reinterpret_cast<unsigned char*>(sm + L.ddep);
   unsigned short* rowoff = reinterpret_cast<unsigned short*>(sm + L.rowoff);
   unsigned char* ancd = reinterpret_cast<unsigned char*>(sm + L.ancd);
@@ -334,83 +330,130 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
   // chain) or the last DOF of the nearest ancestor joint that has DOFs.  The residuals
   // couple a DOF only with its ancestors (a pose target's support is a root-to-frame
   // path; limit, rest and damping terms are diagonal), so J^T J is stored as one row per
-  // DOF over its ancestors and itself, entry (i, j) at rowoff[i] + ddep[j], and factors
+  // DOF over its ancestors and itself, entry (i, j) at rowoff[i] + 1 + ddep[j] (the row's
+  // first slot holds its right-hand side; rows have even lengths), and factors
   // leaves first with no fill-in.  DOF numbering is topological (dpar[c] < c), so a
-  // DOF's ancestors have smaller indices.  One lane builds the tables once per problem.
-  if (tl == 0) {
-    int* lastd = reinterpret_cast<int*>(poseA);  // scratch: last DOF on each joint's path
-    for (int j = 0; j < nj; ++j) {
-      const int pj = parent[j];
-      const int prev = pj >= 0 ? lastd[pj] : -1;
-      const int jt = jtype[j];
-      const int nvj = joint_nv(jt);
-      for (int k = 0; k < nvj; ++k) dpar[idxv[j] + k] = (signed char)(k == 0 ? prev : idxv[j] + k - 1);
-      lastd[j] = nvj ? idxv[j] + nvj - 1 : prev;
-    }
-    int nl = 0, dlev = 0;
+  // DOF's ancestors have smaller indices.
+  // Lane c's ancestors are the DOFs of its joint's proper ancestors and the earlier DOFs of its own.
+  tm.sync();
+  {
     bool bad = false;
+    int dlev = 0, base = 0;
     const int As = L.anc_stride;
-    for (int c = 0; c < nv; ++c) {
-      const int pc = dpar[c];
-      const int dc = pc < 0 ? 0 : ddep[pc] + 1;
-      ddep[c] = (unsigned char)dc;
-      dlev = dc + 1 > dlev ? dc + 1 : dlev;
-      amask[c] = pc < 0 ? 0ull : (amask[pc] | (1ull << pc));
-      if (dc > As) {
-        bad = true;  // deeper than the tree's dof_depth claims: the ancestor table would overflow
-      } else {
+#pragma unroll
+    for (int r = 0; r < lm_rows(T); ++r) {
+      const int c = r * T + tl;
+      const bool in = c < nv;
+      unsigned long long am = 0ull;
+      int dc = 0;
+      if (in) {
+        const int j = cjoint[c], iv = idxv[j];
+        am = (1ull << c) - (1ull << iv);               // this joint's DOFs before c
 #pragma unroll 1
-        for (int a = 0; a + 1 < dc; ++a) ancd[c * As + a] = ancd[pc * As + a];
-        if (pc >= 0) ancd[c * As + dc - 1] = (unsigned char)pc;
+        for (unsigned long long sp = support[j] & ~(1ull << j); sp; sp &= sp - 1ull) {
+          const int i = __ffsll((long long)sp) - 1, ni = joint_nv(jtype[i]);
+          if (ni) am |= ((1ull << ni) - 1ull) << idxv[i];
+        }
+        dc = __popcll(am);
+        ddep[c] = (unsigned char)dc;
+        if (dc > As) {
+          bad = true;  // deeper than the tree's dof_depth claims: the ancestor table would overflow
+        } else {
+          int a = 0;
+#pragma unroll 1
+          for (unsigned long long m = am; m; m &= m - 1ull) ancd[c * As + a++] = (unsigned char)(__ffsll((long long)m) - 1);
+        }
+        dlev = dc + 1 > dlev ? dc + 1 : dlev;
       }
-      rowoff[c] = (unsigned short)nl;
-      nl += dc + 1;
+      int off = in ? (dc + 3) & ~1 : 0;                // row offsets: a scan of the row lengths
+#pragma unroll
+      for (int o = 1; o < T; o <<= 1) {
+        const int x = __shfl_up_sync(tm.mask, off, o, T);
+        if (tl >= o) off += x;
+      }
+      if (in) rowoff[c + 1] = (unsigned short)(base + off);
+      base += __shfl_sync(tm.mask, off, T - 1, T);
     }
-    rowoff[nv] = (unsigned short)nl;
-    misc[0] = (bad || nl > L.n_ent) ? 1 : 0;
-    misc[1] = dlev;
-    // trunk: the largest n <= kTrunkMax such that DOFs 0..n-1 form a chain from the root and
-    // every other DOF descends from DOF n - 1 (a floating base's six DOFs; the top of a serial
-    // chain).  The schedule's last n levels then eliminate n - 1, ..., 0, one DOF each.
-    int ntr = 0;
-#pragma unroll 1
-    for (int n = kF64 ? (nv < kTrunkMax ? nv : kTrunkMax) : 0; n >= 2 && ntr == 0; --n) {
-      bool ok = dpar[0] < 0;
-#pragma unroll 1
-      for (int c = 1; c < n && ok; ++c) ok = dpar[c] == c - 1;
-#pragma unroll 1
-      for (int c = n; c < nv && ok; ++c) ok = ((amask[c] >> (n - 1)) & 1ull) != 0;
-      if (ok) ntr = n;
+    if (tl == 0) rowoff[0] = 0;
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) {
+      const int x = __shfl_xor_sync(tm.mask, dlev, o, T);
+      dlev = x > dlev ? x : dlev;
     }
-    misc[2] = ntr;
+    bad = __any_sync(tm.mask, bad) || base > L.n_ent;
+    if (tl == 0) {
+      misc[0] = bad ? 1 : 0;
+      misc[1] = dlev;
+    }
   }
   tm.sync();
   // level schedule (br_tree_t.dof_sched): every offset it holds must address this
   // problem's factor storage; checked once per team and schedule
   const uint32_t* sched = tree.dof_sched;  // non-null: checked on the host
+  const uint32_t* rsched = sched + (((((5 + (int)sched[0] + 3) & ~3) + 4 * (int)sched[1] + 2 * (int)sched[2]) + 3) & ~3);
   if (sched != sched_ok && !misc[0]) {
-    const int nL0 = rowoff[nv], lim = nL0 + nv;
+    int lim = nv;                                      // the entry schedule's offsets: unpadded rows, then nv slots
+    for (int c = 0; c < nv; ++c) lim += ddep[c] + 1;
     const int nlev = (int)sched[0], ntask = (int)sched[1], nextra = (int)sched[2];
     bool bad = nlev < 0 || nlev > nv || ntask < 0 || nextra < 0 || (int)sched[3] != misc[1];
-    if (!bad) {
+    auto starts_ok = [&](const uint32_t* st, int levs, int last) {
+      bool ok = true;
 #pragma unroll 1
-      for (int l = tl; l <= nlev; l += T) {
-        const int s0 = (int)sched[4 + l];
-        bad |= (l == 0 && s0 != 0) || (l == nlev && s0 != ntask) || s0 < 0 || s0 > ntask ||
-               (l > 0 && s0 < (int)sched[3 + l]);
+      for (int l = tl; l <= levs; l += T) {
+        const int s0 = (int)st[l];
+        ok = ok && !((l == 0 && s0 != 0) || (l == levs && s0 != last) || s0 < 0 || s0 > last ||
+                     (l > 0 && s0 < (int)st[l - 1]));
       }
+      return ok;
+    };
+    if (!bad) {
+      bad |= !starts_ok(sched + 4, nlev, ntask);
       const int toff = (5 + nlev + 3) & ~3;
       const uint4* tk = reinterpret_cast<const uint4*>(sched + toff);
       const uint2* ex = reinterpret_cast<const uint2*>(sched + toff + 4 * ntask);
+#pragma unroll 4
       for (int p = tl; p < ntask; p += T) {
         const uint4 t4 = tk[p];
         bad |= (int)(t4.x & 0xffff) >= lim || (int)(t4.y & 0xffff) >= lim || (int)(t4.y >> 16) >= lim ||
                (int)(t4.z & 0xffff) >= nv || (int)(t4.z >> 16) + (int)(t4.x >> 16) > nextra || (int)t4.w > nv;
       }
-#pragma unroll 1
+#pragma unroll 4
       for (int e = tl; e < nextra; e += T) {
         const uint2 e2 = ex[e];
         bad |= (int)(e2.x & 0xffff) >= lim || (int)(e2.x >> 16) >= lim || (int)e2.y >= nv;
+      }
+    }
+    if (!__any_sync(tm.mask, bad)) {                   // the row schedule: every pair inside the padded rows
+      const int nr = rowoff[nv], nrt = (int)rsched[0], nrx = (int)rsched[1];
+      const int blev = (int)(rsched[2] & 0xffff), ntr = (int)(rsched[2] >> 16);
+      bad = nrt < 0 || nrx < 0 || ntr > kTrunkMax || ntr > nv || blev + ntr != nlev || (int)rsched[3] != nr;
+      if (!bad) {
+        bad |= !starts_ok(rsched + 4, blev, nrt);
+        const uint32_t* rt = rsched + ((5 + nlev + 3) & ~3);
+#pragma unroll 1
+        for (int c = tl; c < nv && ntr > 0; c += T) {  // the trunk is the tree's
+          if (c < ntr) {
+            bad |= ddep[c] != c;
+          } else {
+            const uint32_t w = rt[4 * nrt + nrx + c - ntr];
+            const int k = (int)(w >> 16);
+            bad |= ddep[c] < ntr || ancd[c * L.anc_stride + ntr - 1] != ntr - 1 || k < ntr || k >= nv ||
+                   (int)(w & 0xffff) != rowoff[k < nv ? k : 0];
+          }
+        }
+        auto from_ok = [&](uint32_t c, int delta, int width) {
+          const int so = (int)(c & 0xffff), src = so - delta;
+          return so < nr && (int)(c >> 16) < nv && src >= 0 && !(src & 1) && src + width <= nr;
+        };
+#pragma unroll 1
+        for (int p = tl; p < nrt; p += T) {
+          const uint4 t4 = reinterpret_cast<const uint4*>(rt)[p];
+          const int dst = (int)(t4.x & 0xffff), delta = (int)((t4.x >> 16) & 0xff), n = (int)(t4.x >> 24);
+          const int first = (int)(t4.z & 0xffff), f = (int)((t4.z >> 16) & 0x7fff), width = (t4.z >> 31) ? 4 : 2;
+          bad |= n < 1 || (dst & 1) || dst + width > nr || f > nv || (f > 0 && delta >= width) ||
+                 (n > 2 && ((first & 1) || first + ((n - 1) & ~1) > nrx)) || !from_ok(t4.y, delta, width) || (n > 1 && !from_ok(t4.w, delta, width));
+          for (int e = 2; e < n && !bad; ++e) bad |= !from_ok(rt[4 * nrt + first + e - 2], delta, width);
+        }
       }
     }
     bad = __any_sync(tm.mask, bad);
@@ -725,7 +768,7 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
 #pragma unroll
           for (int r = 0; r < 6; ++r) acc = rfma(Jc[r * nv + u], Jc[r * nv + v], acc);
         }
-        jtj[rowoff[st[u]] + ddep[st[v]]] += acc;  // st ascending: st[u] descends from st[v]
+        jtj[rowoff[st[u]] + 1 + ddep[st[v]]] += acc;  // st ascending: st[u] descends from st[v]
       }
       const R rw[6] = {wp * (R)e[0] * kw[0], wp * (R)e[1] * kw[1], wp * (R)e[2] * kw[2],
                        wo * (R)e[3] * kw[3], wo * (R)e[4] * kw[4], wo * (R)e[5] * kw[5]};
@@ -766,8 +809,8 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
           }
         }
       }
-      jtj[rowoff[c] + ddep[c]] += dg;
-      g[c] = gc;
+      jtj[rowoff[c] + 1 + ddep[c]] += dg;
+      jtj[rowoff[c]] = -gc;
       gg += gc * gc;
     }
 #pragma unroll
@@ -787,10 +830,14 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
   // eliminated together (tasks of the schedule, one lane each), the right-hand side
   // -g is updated in the same tasks (forward substitution), then back substitution
   // runs root first by depth: delta_i = (z_i - sum_a Lm[i][a] delta_anc(i, a)) / D_i.
+  // A task is up to four consecutive entries of one row (its right-hand side the first): the
+  // contributions of one DOF k to them share the factor -l_ki = -m[s] / pivot_k, each entry takes
+  // its contributions in descending k, so the result does not depend on how entries are grouped.
+  // Grouping cut the tasks of a humanoid factorization from 977 (and 621 further contributions)
+  // to 211 and 37 passes of the team to 10; its trunk (the free-flyer's six DOFs) follows in registers.
   auto solve = [&](R damp) -> bool {
     R* Lm = work;
-    R* z = work + nL;
-    {  // Lm = J^T J, 16-byte vectors (both regions start on a 16-byte boundary)
+    {  // Lm = the rows of -g and J^T J, 16-byte vectors (both regions start on a 16-byte boundary)
       using V = typename std::conditional<kF64, double2, float4>::type;
       constexpr int VW = 16 / (int)sizeof(R);
       const int nvec = nL / VW;
@@ -805,26 +852,22 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
     // here fails for it only when the final one would: the outcome of one test at the end).
     bool bad = false;
     for (int i = tl; i < nv; i += T) {
-      z[i] = -g[i];
-      const R piv = jtj[rowoff[i] + ddep[i]] + damp;
+      const R piv = jtj[rowoff[i] + 1 + ddep[i]] + damp;
       bad |= !(piv > (R)0) || !isfinite(piv);
       dinv[i] = rrcp(piv);
     }
     tm.sync();
-    const int nlev = (int)sched[0];
-    const int toff = (5 + nlev + 3) & ~3;
-    const uint4* tasks = reinterpret_cast<const uint4*>(sched + toff);
-    const uint2* extra = reinterpret_cast<const uint2*>(sched + toff + 4 * (int)sched[1]);
+    using V2 = typename std::conditional<kF64, double2, float2>::type;
+    const int nlev = (int)(rsched[2] & 0xffff), ntr = (int)(rsched[2] >> 16);
+    const int last = (int)rsched[0] - 1;
+    const uint4* tasks = reinterpret_cast<const uint4*>(rsched + ((5 + nlev + ntr + 3) & ~3));
+    const uint32_t* extra = reinterpret_cast<const uint32_t*>(tasks + (last + 1));
     // this lane's first task of level l + 1 is loaded during level l (its index clamped to the
     // last task, used only when it lies in level l + 1)
-    const int last = (int)sched[1] - 1;
     int t0 = 0;
     uint4 first = last >= 0 ? __ldg(tasks + (tl < last ? tl : last)) : make_uint4(0u, 0u, 0u, 0u);
-    // the trunk's levels run in registers in the float64 variants only (measured on the
-    // 8,192-problem mix: float64 4.05 -> 4.00 ms, float32 2.76 -> 2.80 ms, outcomes identical)
-    const int ntr = kF64 ? misc[2] : 0;
-    for (int l = 0; l < nlev - ntr; ++l) {
-      const int t1 = (int)__ldg(sched + 5 + l);
+    for (int l = 0; l < nlev; ++l) {
+      const int t1 = (int)__ldg(rsched + 5 + l);
       int p = t0 + tl;
       uint4 nx = p < t1 ? first : make_uint4(0u, 0u, 0u, 0u);
       if (last >= 0) first = __ldg(tasks + (t1 + tl < last ? t1 + tl : last));
@@ -832,37 +875,52 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
       for (; p < t1; p += T) {
         const uint4 tk = nx;                                   // the next pass's task is in flight
         if (p + T < t1) nx = __ldg(tasks + p + T);
-        const int dst = tk.x & 0xffff;
-        R acc = rfma(-Lm[tk.y & 0xffff] * dinv[tk.z & 0xffff], Lm[tk.y >> 16], Lm[dst]);
-        int e = (int)(tk.z >> 16);
-        const int e1 = e + (int)(tk.x >> 16);
-        for (; e + 1 < e1; e += 2) {                           // two records in flight at once
-          const uint2 ea = __ldg(extra + e), eb = __ldg(extra + e + 1);
-          const R a1 = Lm[ea.x & 0xffff] * dinv[ea.y], a2 = Lm[ea.x >> 16];
-          const R b1 = Lm[eb.x & 0xffff] * dinv[eb.y], b2 = Lm[eb.x >> 16];
-          acc = rfma(-a1, a2, acc);
-          acc = rfma(-b1, b2, acc);
+        V2* dst = reinterpret_cast<V2*>(Lm + (tk.x & 0xffff));
+        const int delta = (int)((tk.x >> 16) & 0xff), n = (int)(tk.x >> 24);
+        const bool two = (int)tk.z < 0;
+        V2 a = dst[0], b = a;
+        if (two) b = dst[1];
+        auto add = [&](uint32_t c) {
+          const R* src = Lm + (c & 0xffff);
+          const R f = -src[0] * dinv[c >> 16];
+          const V2* v = reinterpret_cast<const V2*>(src - delta);
+          const V2 x = v[0];
+          a.x = rfma(f, x.x, a.x); a.y = rfma(f, x.y, a.y);
+          if (two) {
+            const V2 y = v[1];
+            b.x = rfma(f, y.x, b.x); b.y = rfma(f, y.y, b.y);
+          }
+        };
+        add(tk.y);
+        if (n > 1) {
+          uint32_t c = tk.w;
+          const uint32_t* e = extra + (tk.z & 0xffff);
+#pragma unroll 1
+          for (int j = 2;; ++j) {                              // the next contribution's word in flight
+            const uint32_t cn = j < n ? __ldg(e + (j - 2)) : 0u;
+            add(c);
+            if (j >= n) break;
+            c = cn;
+          }
         }
-        if (e < e1) {
-          const uint2 ex = __ldg(extra + e);
-          acc = rfma(-Lm[ex.x & 0xffff] * dinv[ex.y], Lm[ex.x >> 16], acc);
-        }
-        Lm[dst] = acc;
-        if (tk.w) {                                            // DOF tk.w - 1's pivot is final
-          const R piv = acc + damp;
+        dst[0] = a;
+        if (two) dst[1] = b;
+        const int f = (int)((tk.z >> 16) & 0x7fff);
+        if (f) {                                               // DOF f - 1's pivot is final
+          const R piv = (delta & 2 ? (delta & 1 ? b.y : b.x) : (delta & 1 ? a.y : a.x)) + damp;
           bad |= !(piv > (R)0) || !isfinite(piv);
-          dinv[tk.w - 1] = rrcp(piv);
+          dinv[f - 1] = rrcp(piv);
         }
       }
       tm.sync();
     }
     if (ntr > 0) {
-      // The trunk's levels in registers: lane t < ne holds the trunk's factor entry t (row i,
-      // column j at t = i (i + 1) / 2 + j: the trunk rows are the first entries of the factor),
-      // lane ne + i the right-hand side z_i; each elimination takes its operands by shuffles
-      // instead of a pass over shared memory and a team synchronisation.  The same operations
-      // in the same order as the schedule's tasks of those levels (one contribution per entry
-      // and level), so the factor is the same to the bit.
+      // The trunk in registers: lane t < ne holds its factor entry t (row i, column j at
+      // t = i (i + 1) / 2 + j), lane ne + i the right-hand side of row i.  First every other DOF's
+      // contribution, in the order of the levels (each entry's operations and their order are those
+      // of updating the trunk level by level: the factor is the same to the bit), then its own
+      // eliminations by shuffles.  Humanoid: its 27 entries were the tasks with five contributions
+      // each that every level waited for.
       const int ne = ntr * (ntr + 1) / 2;
       const bool ent = tl < ne, rhs = !ent && tl < ne + ntr;
       int ri = 0, cj = 0;
@@ -873,8 +931,25 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
       } else if (rhs) {
         ri = tl - ne;
       }
-      R v = ent ? Lm[tl] : rhs ? z[ri] : (R)0;
-      R dk = dinv[ntr - 1];                                    // final since the levels below
+      const int pos = ent ? 1 + cj : 0;
+      R* slot = Lm + rowoff[ri] + pos;
+      R v = *slot;                                             // (lanes beyond carry a copy of DOF 0's)
+      const uint32_t* from = extra + (int)rsched[1];
+      const R* li = Lm + 1 + ri;
+      const R* lj = Lm + pos;
+#pragma unroll 4
+      for (int e = 0; e < nv - ntr; ++e) {
+        const uint32_t w = __ldg(from + e);
+        const int o = (int)(w & 0xffff);
+        v = rfma(-li[o] * dinv[w >> 16], lj[o], v);
+      }
+      R dk;
+      {                                                        // DOF ntr - 1's pivot, now final
+        const R piv = __shfl_sync(tm.mask, v, ne - 1) + damp;
+        bad |= !(piv > (R)0) || !isfinite(piv);
+        dk = rrcp(piv);
+        if (tl == 0) dinv[ntr - 1] = dk;
+      }
 #pragma unroll 1
       for (int k = ntr - 1; k >= 1; --k) {                     // eliminate DOF k
         const int rk = tri(k);
@@ -886,8 +961,7 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
         dk = rrcp(piv);
         if (tl == 0) dinv[k - 1] = dk;
       }
-      if (ent) Lm[tl] = v;
-      else if (rhs) z[ri] = v;
+      if (ent || rhs) *slot = v;
       tm.sync();
     }
     if (__any_sync(tm.mask, bad)) return false;
@@ -901,10 +975,10 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
     for (int r = 0; r < NR; ++r) {
       const int i = tl + T * r;
       const bool in = i < nv;
-      zr[r] = in ? z[i] : (R)0;
+      ror[r] = in ? rowoff[i] + 1 : 1;
+      zr[r] = in ? Lm[ror[r] - 1] : (R)0;
       dvr[r] = in ? dinv[i] : (R)0;
       dr[r] = in ? ddep[i] : -1;
-      ror[r] = in ? rowoff[i] : 0;
     }
     const int ndl = misc[1];
 #pragma unroll 1

@@ -117,6 +117,23 @@ typedef struct br_tree {
  * Offsets index the packed rows (row c starts at sum_{c' < c} (depth(c') + 1), its
  * diagonal at depth(c)) followed by the nv right-hand-side slots.
  *
+ * The row schedule follows (the one the kernel runs; the entries above are checked against the tree and
+ * otherwise unused): at word roff = roundup(toff + 4 tasks + 2 extra, 4), in rows of {right-hand side,
+ * entries by depth} padded to an even length (row c starts at sum_{c' < c} (depth(c') + 3 & ~1)).  The
+ * trunk, the first n <= 6 DOFs when they form a chain from the root that every other DOF descends from
+ * (n = 0 if there are not two), takes no part in its levels.
+ * [0] row tasks, [1] further contributions, [2] levels below the trunk | (n << 16), [3] length of the
+ * rows, [4 .. 4 + levels] first task of each level, then at roff + roundup(5 + all levels, 4) the tasks,
+ * 4 words each:
+ *   {dst | (delta << 16) | (cnt << 24), c_0, first | (f << 16) | (two << 31), c_1 (0 if cnt = 1)}
+ *   for each contribution c_j = s | (k << 16), j < cnt (c_2.. from word `first`, even, of the list that
+ *   follows the tasks, each task's padded to pairs): m[dst + e] -= (m[s] / (pivot_k + damp)) m[s - delta + e],
+ *   e = 0, 1 and, if two, 2, 3; f = c + 1 when the task ends with DOF c's diagonal final (it is
+ *   m[dst + delta]), else 0,
+ * then the further contributions, then, if n > 0, one word row(k) | (k << 16) for each of the nv - n DOFs
+ * below the trunk in the order of their levels: entry e of trunk row i, m[row(i) + e] -=
+ * (m[row(k) + 1 + i] / (pivot_k + damp)) m[row(k) + e].
+ *
  * Writes the schedule to `out` (HOST, `capacity` words) when it fits and returns
  * the number of words it needs, or BR_EINVAL (bad dof_parent) / BR_ETOOBIG (more
  * than 65,535 packed offsets or extra contributions).  Host-only: no device work.
