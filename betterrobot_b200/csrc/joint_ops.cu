@@ -221,9 +221,39 @@ __global__ void __launch_bounds__(32 * kJointOpsWarps) joint_ops_kernel(const br
   if (kVec) cp_async_wait_all();
 }
 
+// *flag = 1 if any row's quaternion norm is further than tol from 1 (a NaN norm is not).  One pass over
+// four floats of each row, bound by latency: 3 us for 16,001 rows of 30 floats, where the norms, the
+// comparison, the reduction and the copy of the answer as tensor operations took 16 us of the GPU and a
+// round trip before the caller's own kernel could start (forward kinematics + joint Jacobians of those
+// configurations: 184 -> 125 us).  The flag may be pinned host memory; it is only written on a violation.
+__global__ void __launch_bounds__(256) check_quaternions_kernel(const float* __restrict__ q, int64_t rows,
+                                                                int32_t row_floats, float tol, int32_t* flag) {
+  bool bad = false;
+  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < rows; b += (int64_t)gridDim.x * blockDim.x) {
+    const float* p = q + b * row_floats;
+    const float x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2), w = __ldg(p + 3);
+    bad = bad || fabsf(sqrtf(x * x + y * y + z * z + w * w) - 1.f) > tol;
+  }
+  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *flag = 1;
+}
+
 }  // namespace br
 
 using namespace br;
+
+extern "C" int br_check_quaternions(const float* quat, int64_t rows, int32_t row_floats, int32_t tol_millionths,
+                                    int32_t* flag, void* stream) {
+  if (rows < 0 || row_floats < 4 || tol_millionths < 0) return BR_EINVAL;
+  if (rows == 0) return BR_OK;
+  if (!quat || !flag) return BR_EINVAL;
+  if (!aligned4(quat) || !aligned4(flag)) return BR_EALIGN;
+  int64_t blocks = (rows + 255) / 256;
+  const int64_t cap = (int64_t)device_info().sms * 8;
+  if (blocks > cap) blocks = cap;
+  check_quaternions_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(quat, rows, row_floats,
+                                                                               1e-6f * (float)tol_millionths, flag);
+  return (int)cudaGetLastError();
+}
 
 extern "C" int br_configuration_op(const br_tree_t* tree, const int32_t* active_joints, int32_t n_active, int32_t op,
                                    const float* a, const float* b, int64_t batch, float* out, void* stream) {

@@ -8,6 +8,7 @@ sm_100a kernels of ``libbr_b200.so``.  Inputs must be float32 CUDA tensors.
 
 from __future__ import annotations
 
+import threading
 from typing import Literal, Sequence
 
 import torch
@@ -31,13 +32,70 @@ def _ref_code(reference) -> int:
 
 def _validate_q(model, q: torch.Tensor, check_quaternion: bool = True) -> None:
     """``_validate_q`` (``forward.py:35-70``) plus the CUDA/float32 requirements of this path."""
+    _validate_form(model, q)
+    if check_quaternion:
+        _QuaternionCheck(model, q, _flat(q)).result()
+
+
+def _validate_form(model, q: torch.Tensor) -> None:
     if q.shape[-1] != model.nq:
         raise ShapeError(f"q has trailing size {q.shape[-1]}, expected model.nq={model.nq}")
     _lib.require_cuda(q)
     if q.dtype != torch.float32:
         raise DtypeMismatchError(f"q.dtype={q.dtype}; the sm_100a path computes in float32")
-    if check_quaternion and model.njoints >= 2 and model.joint_models[1].kind == "free_flyer" and q.numel():
-        norm = q[..., 3:7].norm(dim=-1)
+
+
+class _Answer(threading.local):
+    """Per thread and device: a pinned flag and the event after the kernel that may write it."""
+
+    def __init__(self):
+        self.by_device: dict = {}
+
+    def get(self, index: int):
+        a = self.by_device.get(index)
+        if a is None:
+            a = self.by_device[index] = (torch.zeros(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event())
+        else:
+            a[1].synchronize()  # done already, unless an exception cut the last check short
+        return a
+
+
+_answer = _Answer()
+# The kernel flags a little more than the check refuses, so that its rounding decides nothing.
+_QUAT_FLAG_MILLIONTHS = int(_QUAT_NORM_TOL * 1e6) - 10
+
+
+class _QuaternionCheck:
+    """The free-flyer quaternion check of a batch: launched here, waited for in ``result``.
+
+    One kernel writes a pinned flag, and the host waits for that kernel alone, so work launched in
+    between runs on meanwhile."""
+
+    def __init__(self, model, q: torch.Tensor, qf: torch.Tensor):
+        self.q = None
+        if model.njoints < 2 or model.joint_models[1].kind != "free_flyer" or not q.numel():
+            return
+        self.q = q
+        with torch.cuda.device(q.device):
+            if torch.cuda.is_current_stream_capturing():
+                self.decide()  # refused by the capture, as any wait is
+                return
+            self.flag, self.event = _answer.get(q.device.index)
+            self.flag[0] = 0
+            stream = torch.cuda.current_stream()
+            _lib.call("br_check_quaternions", qf.data_ptr() + 12, qf.shape[0], qf.shape[1], _QUAT_FLAG_MILLIONTHS,
+                      self.flag.data_ptr(), stream.cuda_stream)
+            self.event.record(stream)
+
+    def result(self) -> None:
+        if self.q is None:
+            return
+        self.event.synchronize()
+        if self.flag[0]:
+            self.decide()
+
+    def decide(self) -> None:
+        norm = self.q[..., 3:7].norm(dim=-1)
         if bool(((norm - 1.0).abs() > _QUAT_NORM_TOL).any()):
             raise QuaternionNormError(
                 f"free-flyer quaternion norm outside [{1 - _QUAT_NORM_TOL}, {1 + _QUAT_NORM_TOL}] "
@@ -57,9 +115,10 @@ def forward_kinematics(model, q_or_data, *, compute_frames: bool = False, backen
     else:
         q = q_or_data
         data = Data(q=q)
-    _validate_q(model, q, check_quaternion)
+    _validate_form(model, q)
     batch = tuple(q.shape[:-1])
     qf = _flat(q)
+    check = _QuaternionCheck(model, q, qf) if check_quaternion else None
     B = qf.shape[0]
     dt = device_tree(model, q.device)
     oMi = torch.empty(B, model.njoints, 7, device=q.device, dtype=torch.float32)
@@ -85,6 +144,8 @@ def forward_kinematics(model, q_or_data, *, compute_frames: bool = False, backen
                 ids = (_lib.c_int32 * nf)(*range(nf))
             _lib.call("br_forward_kinematics", dt.ptr, qf.data_ptr(), B, oMi.data_ptr(), liMi.data_ptr(),
                       ids, nf, frames.data_ptr() if frames is not None else None, _lib.stream_ptr())
+    if check is not None:
+        check.result()
     object.__setattr__(data, "joint_pose_world", oMi.reshape(*batch, model.njoints, 7))
     object.__setattr__(data, "joint_pose_local", liMi.reshape(*batch, model.njoints, 7))
     object.__setattr__(data, "joint_jacobians", None)

@@ -375,6 +375,14 @@ BR_API int br_trajopt_solve(const br_tree_t* tree, int32_t frame_id, int64_t n_t
 BR_API int br_configuration_op(const br_tree_t* tree, const int32_t* active_joints, int32_t n_active, int32_t op,
                                const float* a, const float* b, int64_t batch, float* out, void* stream);
 
+/*
+ * Sets *flag (DEVICE or pinned host memory, never cleared) to 1 if the norm of any of the `rows`
+ * quaternions, row_floats apart, is further than 1e-6 * tol_millionths from 1: the free-flyer check of
+ * src/better_robot/kinematics/forward.py:35-70.
+ */
+BR_API int br_check_quaternions(const float* quat, int64_t rows, int32_t row_floats, int32_t tol_millionths,
+                                int32_t* flag, void* stream);
+
 /* ==== batched SE3 / SO3 primitives (the LieOps seam) ====================== */
 /*
  * Replaces the per-op LieOps protocol (src/better_robot/backends/protocol.py:27-51)
