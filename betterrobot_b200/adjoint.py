@@ -28,19 +28,6 @@ from .exceptions import ShapeError
 from .kinematics import _validate_q
 from .tree import device_tree
 
-_IDS: dict = {}
-
-
-def _ids(frame_ids: tuple):
-    """The frame ids as a ctypes array, built once per id tuple."""
-    arr = _IDS.get(frame_ids)
-    if arr is None:
-        if len(_IDS) >= 256:
-            _IDS.clear()
-        arr = _IDS[frame_ids] = (_lib.c_int32 * len(frame_ids))(*frame_ids)
-    return arr
-
-
 def path_slots(arrays, frame_ids: tuple) -> int:
     """Most joints on one root-to-leaf path that hold a waiting wrench in the adjoint's walk: in the tree
     pruned to the frames' ancestors, those with a child and a frame of their own or a second child.
@@ -65,20 +52,12 @@ def path_slots(arrays, frame_ids: tuple) -> int:
     return n
 
 
-def _on_device(device, fn) -> None:
-    """Run ``fn(stream)`` with ``device`` current (no context switch when it already is)."""
-    if device.index == torch.cuda.current_device():
-        fn(torch.cuda.current_stream().cuda_stream)
-    else:
-        with torch.cuda.device(device):
-            fn(torch.cuda.current_stream().cuda_stream)
-
-
 def _loss_only(model, q, frame_ids, targets, weights):
     loss = torch.empty(q.shape[0], device=q.device, dtype=torch.float32)
-    _on_device(q.device, lambda s: _lib.call(
-        "br_pose_loss", device_tree(model, q.device).ptr, q.data_ptr(), q.shape[0], _ids(frame_ids), len(frame_ids),
-        targets.data_ptr(), weights.data_ptr(), int(weights.dim() == 2), loss.data_ptr(), None, s))
+    with _lib.on(q.device):
+        _lib.call("br_pose_loss", device_tree(model, q.device).ptr, q.data_ptr(), q.shape[0],
+                  _lib.id_array(frame_ids), len(frame_ids), targets.data_ptr(), weights.data_ptr(),
+                  int(weights.dim() == 2), loss.data_ptr(), None, _lib.stream_ptr())
     return loss
 
 
@@ -89,10 +68,11 @@ class _PoseLoss(torch.autograd.Function):
             return _loss_only(model, q, frame_ids, targets, weights)
         loss = torch.empty(q.shape[0], device=q.device, dtype=torch.float32)
         unit = torch.empty_like(q)
-        _on_device(q.device, lambda s: _lib.call(
-            "br_pose_loss_value_grad", device_tree(model, q.device).ptr, q.data_ptr(), q.shape[0], _ids(frame_ids),
-            len(frame_ids), targets.data_ptr(), weights.data_ptr(), int(weights.dim() == 2),
-            path_slots(device_tree(model, q.device).arrays, frame_ids), loss.data_ptr(), unit.data_ptr(), s))
+        dt = device_tree(model, q.device)
+        with _lib.on(q.device):
+            _lib.call("br_pose_loss_value_grad", dt.ptr, q.data_ptr(), q.shape[0], _lib.id_array(frame_ids),
+                      len(frame_ids), targets.data_ptr(), weights.data_ptr(), int(weights.dim() == 2),
+                      path_slots(dt.arrays, frame_ids), loss.data_ptr(), unit.data_ptr(), _lib.stream_ptr())
         # the inputs too: changing one in place before the backward stays an error
         ctx.save_for_backward(q, targets, weights, unit)
         return loss
@@ -104,9 +84,9 @@ class _PoseLoss(torch.autograd.Function):
         if g.stride(0) not in (0, 1):
             g = g.contiguous()
         grad_q = torch.empty_like(unit)
-        _on_device(unit.device, lambda s: _lib.call(
-            "br_scale_rows", unit.data_ptr(), g.data_ptr(), g.stride(0), unit.shape[0], unit.shape[1],
-            grad_q.data_ptr(), s))
+        with _lib.on(unit.device):
+            _lib.call("br_scale_rows", unit.data_ptr(), g.data_ptr(), g.stride(0), unit.shape[0], unit.shape[1],
+                      grad_q.data_ptr(), _lib.stream_ptr())
         return grad_q, None, None, None, None, None
 
 

@@ -24,19 +24,28 @@ def _check(t: torch.Tensor, n: int, name: str):
         raise DtypeMismatchError(f"{name}.dtype={t.dtype}; the sm_100a path computes in float32")
 
 
+def _flat(t, batch):
+    """The rows of ``t`` broadcast to ``batch``, contiguous."""
+    if t.shape[:-1] == batch and t.shape[-1] and t.is_contiguous():
+        return t
+    return t.expand(*batch, t.shape[-1]).reshape(-1, t.shape[-1]).contiguous()
+
+
 def _run(model, op, a, b, out_dim, out=None):
-    batch = torch.broadcast_shapes(a.shape[:-1], b.shape[:-1])
-    af = a.expand(*batch, a.shape[-1]).reshape(-1, a.shape[-1]).contiguous()
-    bf = b.expand(*batch, b.shape[-1]).reshape(-1, b.shape[-1]).contiguous()
+    batch = a.shape[:-1]
+    if batch != b.shape[:-1]:
+        batch = torch.broadcast_shapes(batch, b.shape[:-1])
+    af, bf = _flat(a, batch), _flat(b, batch)
+    n = batch.numel()
     if out is None:
-        out = torch.empty(af.shape[0], out_dim, device=a.device, dtype=torch.float32)
-    elif (out.shape[-1] != out_dim or out.numel() != af.shape[0] * out_dim or not out.is_contiguous()
+        out = torch.empty(n, out_dim, device=a.device, dtype=torch.float32)
+    elif (out.shape[-1] != out_dim or out.numel() != n * out_dim or not out.is_contiguous()
           or out.dtype != torch.float32 or out.device != a.device):
-        raise ShapeError(f"out must be a contiguous float32 ({af.shape[0]}, {out_dim}) tensor on {a.device}")
+        raise ShapeError(f"out must be a contiguous float32 ({n}, {out_dim}) tensor on {a.device}")
     dt = device_tree(model, a.device)
-    with torch.cuda.device(a.device):
+    with _lib.on(a.device):
         _lib.call("br_configuration_op", dt.ptr, dt.active.data_ptr(), dt.n_active, op, af.data_ptr(), bf.data_ptr(),
-                  af.shape[0], out.data_ptr(), _lib.stream_ptr())
+                  n, out.data_ptr(), _lib.stream_ptr())
     return out.reshape(*batch, out_dim)
 
 

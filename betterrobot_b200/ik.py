@@ -26,6 +26,7 @@ from .tree import device_tree
 OPT_LM, OPT_GN = 0, 1
 MAX_CLASSES, MAX_TARGETS = 8, 8
 SCRATCH_BYTES = 16
+HOST_FILL_FLOATS = 16384
 
 
 @dataclass
@@ -164,6 +165,13 @@ class PackedIK:
     def __init__(self, models: Sequence, frame_ids: Sequence, n_targets: Sequence, q_rest: Sequence | None = None,
                  team_sizes: Sequence[int] | None = None, device="cuda", warps_per_cta: int = 4,
                  with_residual: bool = False, target_kinds: Sequence | None = None):
+        self._build(models, frame_ids, n_targets, q_rest, team_sizes, device, warps_per_cta, with_residual,
+                    target_kinds, True)
+
+    def _build(self, models, frame_ids, n_targets, q_rest, team_sizes, device, warps_per_cta, with_residual,
+               target_kinds, fill: bool) -> None:
+        """``fill``: the identity targets and zero start configurations of a plan that is solved before
+        ``set_inputs`` are written."""
         if not 1 <= len(models) <= MAX_CLASSES:
             raise ShapeError(f"1..{MAX_CLASSES} robot classes per launch, got {len(models)}")
         self.device = torch.device(device)
@@ -171,10 +179,12 @@ class PackedIK:
             self.device = torch.device("cuda", torch.cuda.current_device())
         self.models = list(models)
         self.C = len(models)
-        self.counts = [int(np.asarray(n).shape[0]) for n in n_targets]
-        self.P = sum(self.counts)
-        self.K = max(int(np.asarray(f).shape[1]) for f in frame_ids)
-        if self.K > MAX_TARGETS:
+        n_targets = [np.asarray(n, np.int32) for n in n_targets]
+        frame_ids = [np.asarray(f, np.int32) for f in frame_ids]
+        self.counts = [int(n.shape[0]) for n in n_targets]
+        P = self.P = sum(self.counts)
+        K = self.K = max(int(f.shape[1]) for f in frame_ids)
+        if K > MAX_TARGETS:
             raise ShapeError(f"at most {MAX_TARGETS} targets per problem")
         self.team = [int(t) for t in (team_sizes or [default_team_size(m) for m in models])]
         for m, t in zip(models, self.team):
@@ -183,112 +193,156 @@ class PackedIK:
         self.trees = [device_tree(m, self.device) for m in models]
         self.warps_per_cta = warps_per_cta
         # per-problem layout: classes contiguous, in class order
-        self.class_start = np.cumsum([0] + self.counts)[:-1]
-        nq = np.concatenate([np.full(n, m.nq, np.int64) for n, m in zip(self.counts, models)])
+        starts, q_total = [0], 0
+        for n, m in zip(self.counts, models):
+            starts.append(starts[-1] + n)
+            q_total += n * m.nq
+        self.class_start = np.array(starts[:-1])
+        self.q_total = q_total
+        kinds = self._kinds_of(target_kinds) if target_kinds is not None else None
+        rest = [torch.as_tensor(m.q_neutral if q_rest is None or q_rest[c] is None else q_rest[c],
+                                dtype=torch.float32).detach().reshape(-1, m.nq) for c, m in enumerate(models)]
+        # Every table of the plan lies in one int32 array and goes up in one copy, and so do the rest
+        # configurations up to 64 KB; larger ones are broadcast on the device.  (Made and copied one by one,
+        # with the fills of the buffers, they took 350 of a single solve's 480 us.)
+        host_rest = q_total <= HOST_FILL_FLOATS and not any(r.is_cuda for r in rest)
+        self._sections, o = {}, SCRATCH_BYTES // 4
+        self._sections["scratch"] = (0, o, None, (o,))
+        for name, n, dtype, shape in (
+                ("order", P, None, (P,)), ("items", 3 * P, None, (3 * P,)), ("n_targets_t", P, None, (P,)),
+                ("frames_t", P * K, None, (P, K)), ("q_offset", 2 * P + 2, torch.int64, (P + 1,)),
+                ("r_offset", 2 * P + 2, torch.int64, (P + 1,)),
+                ("kinds", 0 if kinds is None else P * K, None, (P, K)),
+                ("q_rest", q_total if host_rest else 0, torch.float32, (q_total,))):
+            self._sections[name] = (o, n, dtype, shape)
+            o += (n + 3) & ~3
+        host = np.zeros(o, np.int32)
+
+        def part(name, dtype=np.int32):
+            o, n = self._sections[name][:2]
+            return host[o:o + n].view(dtype)
+
+        nt_all, fr = part("n_targets_t"), part("frames_t").reshape(P, K)
         # P + 1 offsets (the last one is the total), so a class with no problems indexes in range
-        self.q_offset_np = np.concatenate([[0], np.cumsum(nq)]).astype(np.int64)
-        self.q_total = int(nq.sum())
-        nt_all = np.concatenate([np.asarray(n, np.int32) for n in n_targets])
-        if (nt_all < 1).any() or (nt_all > self.K).any():
-            raise ShapeError("each problem needs 1..K targets")
-        fr = np.zeros((self.P, self.K), np.int32)
-        for c in range(self.C):
-            f = np.asarray(frame_ids[c], np.int32)
-            if f.size and (f.min() < 0 or f.max() >= models[c].nframes):
+        self.q_offset_np, self.r_offset_np = part("q_offset", np.int64), part("r_offset", np.int64)
+        self.r_dim = np.empty(P, np.int64)
+        for c, (m, n, f) in enumerate(zip(models, n_targets, frame_ids)):
+            s0, s1 = starts[c], starts[c + 1]
+            if n.size and (n.min() < 1 or n.max() > K):
+                raise ShapeError("each problem needs 1..K targets")
+            if f.size and (f.min() < 0 or f.max() >= m.nframes):
                 raise ShapeError(f"class {c}: frame id out of range")
-            s0 = self.class_start[c]
-            fr[s0:s0 + self.counts[c], :f.shape[1]] = f
-        kinds = np.zeros((self.P, self.K), np.int32)
-        if target_kinds is not None:
-            for c in range(self.C):
-                if target_kinds[c] is None:
-                    continue
-                k = np.asarray([TARGET_KINDS[x] if isinstance(x, str) else int(x)
-                                for x in np.asarray(target_kinds[c]).reshape(-1)], np.int32)
-                k = k.reshape(np.asarray(target_kinds[c]).shape)
-                if ((k < 0) | (k > 2)).any():
-                    raise ShapeError("target kinds are 'pose', 'position' or 'orientation'")
-                s0 = self.class_start[c]
-                kinds[s0:s0 + self.counts[c], :k.shape[-1]] = np.broadcast_to(k, (self.counts[c], k.shape[-1]))
-        rows = np.where(kinds == 0, 6, 3) * (np.arange(self.K)[None, :] < nt_all[:, None])
-        dims = []
-        for c, m in enumerate(models):
-            s0 = self.class_start[c]
-            dims.append(rows[s0:s0 + self.counts[c]].sum(-1) + 2 * m.nq + m.nv)
-        rdim = np.concatenate(dims)
-        self.r_offset_np = np.concatenate([[0], np.cumsum(rdim)]).astype(np.int64)
-        self.r_dim = rdim
+            nt_all[s0:s1] = n
+            fr[s0:s1, :f.shape[1]] = f
+            self.q_offset_np[s0 + 1:s1 + 1] = m.nq
+            if kinds is None:
+                rows = 6 * n
+            else:
+                rows = (np.where(kinds[s0:s1] == 0, 6, 3) * (np.arange(K)[None, :] < n[:, None])).sum(-1)
+            self.r_dim[s0:s1] = rows + (2 * m.nq + m.nv)
+        np.cumsum(self.q_offset_np, out=self.q_offset_np)
+        np.cumsum(self.r_dim, out=self.r_offset_np[1:])
         # work items: heaviest classes first, and inside a class the problems with the fewest
         # targets first (they run the most iterations: a less constrained problem's rest term
         # settles slowly), so the longest solves start early and the launch's tail is short
-        cost = [m.nv ** 2 * (1 + self.K) for m in models]
-        order, items = [], []
-        slot = 0
+        cost = [m.nv ** 2 * (1 + K) for m in models]
+        order, items, slot = part("order"), part("items").reshape(P, 3), 0  # item: (slot, problems, class)
+        items[:, 0] = np.arange(P, dtype=np.int32)
+        items[:, 1] = 1  # one problem per 32-lane team
         for c in sorted(range(self.C), key=lambda k: -cost[k]):
-            per = 32 // self.team[c]
-            s0 = int(self.class_start[c])
-            idx = s0 + np.argsort(nt_all[s0:s0 + self.counts[c]], kind="stable")
-            order.append(idx)
-            for s in range(0, self.counts[c], per):
-                items.append((slot + s, min(per, self.counts[c] - s), c))
-            slot += self.counts[c]
+            n = self.counts[c]
+            order[slot:slot + n] = np.argsort(n_targets[c], kind="stable")
+            order[slot:slot + n] += starts[c]
+            items[slot:slot + n, 2] = c
+            slot += n
+        self.n_items = P
+        if kinds is not None:
+            part("kinds").reshape(P, K)[...] = kinds
         dev = self.device
-        self.order = torch.from_numpy(np.concatenate(order).astype(np.int32)).to(dev)
-        self.items = torch.tensor(items, dtype=torch.int32, device=dev).reshape(-1)
-        self.n_items = len(items)
-        self.n_targets_t = torch.from_numpy(nt_all).to(dev)
-        self.frames_t = torch.from_numpy(fr).to(dev)
-        self.q_offset = torch.from_numpy(self.q_offset_np).to(dev)
-        self.r_offset = torch.from_numpy(self.r_offset_np).to(dev)
-        self.kinds = torch.from_numpy(kinds).to(dev) if kinds.any() else None
-        self.targets = torch.zeros(self.P, self.K, 7, device=dev)
-        self.targets[..., 6] = 1.0
-        self.x0 = torch.zeros(self.q_total, device=dev)
-        self.q_rest = torch.zeros(self.q_total, device=dev)
-        for c, m in enumerate(models):
-            qr = (m.q_neutral if q_rest is None or q_rest[c] is None else q_rest[c])
-            qr = torch.as_tensor(qr, dtype=torch.float32).reshape(-1, m.nq)
-            s0 = int(self.q_offset_np[self.class_start[c]])
-            self.q_rest[s0:s0 + self.counts[c] * m.nq] = qr.to(dev).expand(self.counts[c], m.nq).reshape(-1)
-        self.x = torch.empty(self.q_total, device=dev)
-        self.iters = torch.empty(self.P, dtype=torch.int32, device=dev)
-        self.status = torch.empty(self.P, dtype=torch.int32, device=dev)
-        self.cost = torch.empty(self.P, device=dev)
+        x0s = [int(self.q_offset_np[s]) for s in starts]
+        if host_rest:
+            qr = part("q_rest", np.float32)
+            for c, m in enumerate(models):
+                qr[x0s[c]:x0s[c + 1]].reshape(-1, m.nq)[...] = rest[c].expand(self.counts[c], m.nq).numpy()
+        self._tables = torch.from_numpy(host).to(dev, non_blocking=True)
+        if not host_rest:
+            self.q_rest = torch.empty(q_total, device=dev)
+            for c, m in enumerate(models):
+                self.q_rest[x0s[c]:x0s[c + 1]].view(-1, m.nq).copy_(rest[c].to(dev).expand(self.counts[c], m.nq))
+        if kinds is None:
+            self.kinds = None
+        self.targets = torch.empty(P, K, 7, device=dev)
+        self.x0 = torch.empty(q_total, device=dev)
+        if fill:
+            self.targets.zero_()
+            self.targets[..., 6] = 1.0
+            self.x0.zero_()
+        self.x = torch.empty(q_total, device=dev)
+        self.verdict = torch.empty(2, P, dtype=torch.int32, device=dev)  # iterations, status
+        self.iters, self.status = self.verdict.unbind()
+        self.cost = torch.empty(P, device=dev)
         # fixed layout per problem: target rows, 2 nq limit rows, nv rest rows (zero when unused)
-        self.residual = torch.zeros(int(rdim.sum()), device=dev) if with_residual else None
-        self.scratch = torch.zeros(SCRATCH_BYTES // 4, dtype=torch.int32, device=dev)
+        self.residual = torch.zeros(int(self.r_offset_np[-1]), device=dev) if with_residual else None
         # ctypes structs (kept alive on the object)
         self._trees = (BrTree * self.C)(*[t.struct for t in self.trees])
         self._teams = (c_int32 * self.C)(*self.team)
+        base = self._tables.data_ptr()
+        at = {name: base + 4 * sec[0] for name, sec in self._sections.items()}
         b = IKBatch()
-        b.n_problems, b.max_targets, b.n_classes, b.n_items = self.P, self.K, self.C, self.n_items
-        b.trees = ctypes.cast(self._trees, ctypes.POINTER(BrTree))
-        b.team_size = ctypes.cast(self._teams, ctypes.POINTER(c_int32))
-        b.items, b.order = self.items.data_ptr(), self.order.data_ptr()
-        b.n_targets, b.frames = self.n_targets_t.data_ptr(), self.frames_t.data_ptr()
-        b.targets, b.q_offset = self.targets.data_ptr(), self.q_offset.data_ptr()
-        b.x0, b.q_rest = self.x0.data_ptr(), self.q_rest.data_ptr()
-        b.r_offset = self.r_offset.data_ptr()
-        b.target_kind = self.kinds.data_ptr() if self.kinds is not None else None
-        self._batch = b
+        b.n_problems, b.max_targets, b.n_classes, b.n_items = P, K, self.C, self.n_items
+        b.trees, b.team_size = self._trees, self._teams
+        b.items, b.order = at["items"], at["order"]
+        b.n_targets, b.frames = at["n_targets_t"], at["frames_t"]
+        b.targets, b.q_offset = self.targets.data_ptr(), at["q_offset"]
+        b.x0, b.q_rest = self.x0.data_ptr(), at["q_rest"] if host_rest else self.q_rest.data_ptr()
+        b.r_offset = at["r_offset"]
+        b.target_kind = at["kinds"] if kinds is not None else None
+        self._batch, self._scratch = b, base
         r = IKResultBuf()
         r.x, r.iters, r.status, r.cost = self.x.data_ptr(), self.iters.data_ptr(), self.status.data_ptr(), \
             self.cost.data_ptr()
         r.residual = self.residual.data_ptr() if self.residual is not None else None
         self._result = r
 
+    def _kinds_of(self, target_kinds):
+        """Target kinds of every problem ``(P, K)``, None when all are poses."""
+        kinds = np.zeros((self.P, self.K), np.int32)
+        for c in range(self.C):
+            if target_kinds[c] is None:
+                continue
+            k = np.asarray([TARGET_KINDS[x] if isinstance(x, str) else int(x)
+                            for x in np.asarray(target_kinds[c]).reshape(-1)], np.int32)
+            k = k.reshape(np.asarray(target_kinds[c]).shape)
+            if ((k < 0) | (k > 2)).any():
+                raise ShapeError("target kinds are 'pose', 'position' or 'orientation'")
+            s0 = self.class_start[c]
+            kinds[s0:s0 + self.counts[c], :k.shape[-1]] = np.broadcast_to(k, (self.counts[c], k.shape[-1]))
+        return kinds if kinds.any() else None
+
+    def __getattr__(self, name):
+        """The device tables as tensors, views of the one buffer, made when asked for."""
+        sec = self.__dict__.get("_sections", {}).get(name)
+        if sec is None:
+            raise AttributeError(name)
+        o, n, dtype, shape = sec
+        t = self._tables[o:o + n]
+        t = (t if dtype is None else t.view(dtype)).view(shape)
+        self.__dict__[name] = t
+        return t
+
     def set_inputs(self, targets: Sequence, q0: Sequence) -> None:
         """Copy per-class targets (P_c, K_c, 7) and start configurations (P_c, nq_c) into the device buffers."""
         for c, m in enumerate(self.models):
             s0, n = int(self.class_start[c]), self.counts[c]
-            t = torch.as_tensor(targets[c], dtype=torch.float32)
+            t = torch.as_tensor(targets[c], dtype=torch.float32).detach()
             self.targets[s0:s0 + n, :t.shape[1]].copy_(t, non_blocking=True)
             o = int(self.q_offset_np[s0])
-            self.x0[o:o + n * m.nq].copy_(torch.as_tensor(q0[c], dtype=torch.float32).reshape(-1), non_blocking=True)
+            self.x0[o:o + n * m.nq].copy_(torch.as_tensor(q0[c], dtype=torch.float32).detach().reshape(-1),
+                                                 non_blocking=True)
 
     def solve(self, settings: IKSettings, stream: int | None = None) -> None:
         _lib.call("br_lm_solve", ctypes.byref(self._batch), ctypes.byref(settings), ctypes.byref(self._result),
-                  self.warps_per_cta, self.scratch.data_ptr(), SCRATCH_BYTES,
+                  self.warps_per_cta, self._scratch, SCRATCH_BYTES,
                   stream if stream is not None else _lib.stream_ptr(self.device))
 
     def capture(self, settings: IKSettings) -> "torch.cuda.CUDAGraph":
@@ -333,6 +387,15 @@ def solve_ik_batched(model, frame_ids, targets: torch.Tensor, initial_q: torch.T
     ``src/better_robot/residuals/pose.py:58-195``.  With ``with_residual`` the stacked
     residual has 6 rows per pose target and 3 per position / orientation target.
     """
+    pk, res = _solve_one_class(model, frame_ids, targets, initial_q, cost_cfg, optimizer_cfg, n_targets,
+                               with_residual, team_size, warps_per_cta, target_kinds)
+    return BatchIKResult(q=pk.q_of(0), iters=pk.iters, converged=(pk.status & 0xFF) == 0, status=pk.status,
+                         cost=pk.cost, residual=res)
+
+
+def _solve_one_class(model, frame_ids, targets, initial_q, cost_cfg=None, optimizer_cfg=None, n_targets=None,
+                     with_residual=False, team_size=None, warps_per_cta=4, target_kinds=None):
+    """The solved ``PackedIK`` and its stacked residual (arguments of ``solve_ik_batched``)."""
     cost_cfg = cost_cfg or IKCostConfig()
     optimizer_cfg = optimizer_cfg or OptimizerConfig()
     if initial_q.dim() != 2 or initial_q.shape[-1] != model.nq:
@@ -347,17 +410,19 @@ def solve_ik_batched(model, frame_ids, targets: torch.Tensor, initial_q: torch.T
         raise ShapeError(f"targets must be ({P}, {K}, 7), got {tuple(targets.shape)}")
     nt = np.full(P, K, np.int32) if n_targets is None else np.asarray(n_targets, np.int32)
     qr = [cost_cfg.q_rest] if cost_cfg.q_rest is not None else None
-    pk = PackedIK([model], [fr], [nt], q_rest=qr, team_sizes=[team_size or default_team_size(model)],
-                  device=initial_q.device, warps_per_cta=warps_per_cta, with_residual=with_residual,
-                  target_kinds=None if target_kinds is None else [target_kinds])
+    pk = PackedIK.__new__(PackedIK)
+    pk._build([model], [fr], [nt], qr, [team_size or default_team_size(model)], initial_q.device, warps_per_cta,
+              with_residual, None if target_kinds is None else [target_kinds], False)
     pk.set_inputs([targets], [initial_q])
-    with torch.cuda.device(initial_q.device):
+    with _lib.on(initial_q.device):
         pk.solve(settings_from(cost_cfg, optimizer_cfg))
     res = None
     if with_residual:
         # the reference's CostStack has a limit / rest block only when its weight is > 0
         # (tasks/ik.py:200-205): drop the unused blocks of the fixed device layout
         def stack_rows(r: torch.Tensor) -> torch.Tensor:
+            if cost_cfg.limit_weight > 0.0 and cost_cfg.rest_weight > 0.0:
+                return r
             nt_rows = r.shape[-1] - 2 * model.nq - model.nv
             parts = [r[..., :nt_rows]]
             if cost_cfg.limit_weight > 0.0:
@@ -370,8 +435,7 @@ def solve_ik_batched(model, frame_ids, targets: torch.Tensor, initial_q: torch.T
         else:
             res = (stack_rows(pk.residual.view(P, -1)) if (pk.r_dim == pk.r_dim[0]).all()
                    else [stack_rows(r) for r in torch.split(pk.residual, [int(d) for d in pk.r_dim])])
-    return BatchIKResult(q=pk.q_of(0), iters=pk.iters, converged=(pk.status & 0xFF) == 0, status=pk.status,
-                         cost=pk.cost, residual=res)
+    return pk, res
 
 
 def solve_ik(model, targets: dict, *, initial_q: torch.Tensor | None = None, cost_cfg: IKCostConfig | None = None,
@@ -390,7 +454,6 @@ def solve_ik(model, targets: dict, *, initial_q: torch.Tensor | None = None, cos
         raise ShapeError("solve_ik needs at least one target")
     fids = [model.frame_id(n) for n in names]
     T = torch.stack([torch.as_tensor(targets[n], dtype=torch.float32).reshape(7) for n in names]).to(dev)
-    out = solve_ik_batched(model, fids, T[None], x0, cost_cfg=cost_cfg, optimizer_cfg=optimizer_cfg,
-                           with_residual=True)
-    return IKResult(q=out.q[0], residual=out.residual[0], iters=int(out.iters[0]), converged=bool(out.converged[0]),
-                    model=model)
+    pk, residual = _solve_one_class(model, fids, T[None], x0, cost_cfg, optimizer_cfg, with_residual=True)
+    (iters,), (status,) = pk.verdict.tolist()
+    return IKResult(q=pk.x, residual=residual[0], iters=iters, converged=(status & 0xFF) == 0, model=model)

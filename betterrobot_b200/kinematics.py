@@ -76,7 +76,7 @@ class _QuaternionCheck:
         if model.njoints < 2 or model.joint_models[1].kind != "free_flyer" or not q.numel():
             return
         self.q = q
-        with torch.cuda.device(q.device):
+        with _lib.on(q.device):
             if torch.cuda.is_current_stream_capturing():
                 self.decide()  # refused by the capture, as any wait is
                 return
@@ -103,6 +103,8 @@ class _QuaternionCheck:
 
 
 def _flat(q: torch.Tensor) -> torch.Tensor:
+    if q.dim() == 2 and q.shape[1] and q.is_contiguous():
+        return q
     return q.reshape(-1, q.shape[-1]).contiguous()
 
 
@@ -121,7 +123,7 @@ def forward_kinematics(model, q_or_data, *, compute_frames: bool = False, backen
     check = _QuaternionCheck(model, q, qf) if check_quaternion else None
     B = qf.shape[0]
     dt = device_tree(model, q.device)
-    oMi = torch.empty(B, model.njoints, 7, device=q.device, dtype=torch.float32)
+    oMi = torch.empty((*batch, model.njoints, 7), device=q.device, dtype=torch.float32)
     liMi = torch.empty_like(oMi)
     frames = None
     nf = 0
@@ -129,7 +131,7 @@ def forward_kinematics(model, q_or_data, *, compute_frames: bool = False, backen
     if compute_frames:
         nf = int(model.nframes)
         frames = torch.empty(B, nf, 7, device=q.device, dtype=torch.float32)
-    with torch.cuda.device(q.device):
+    with _lib.on(q.device):
         if compute_frames and nf > 64:
             _lib.call("br_forward_kinematics", dt.ptr, qf.data_ptr(), B, oMi.data_ptr(), liMi.data_ptr(),
                       None, 0, None, _lib.stream_ptr())
@@ -141,13 +143,13 @@ def forward_kinematics(model, q_or_data, *, compute_frames: bool = False, backen
                 frames[:, s:s + len(ids)] = part
         else:
             if compute_frames:
-                ids = (_lib.c_int32 * nf)(*range(nf))
+                ids = _lib.id_array(tuple(range(nf)))
             _lib.call("br_forward_kinematics", dt.ptr, qf.data_ptr(), B, oMi.data_ptr(), liMi.data_ptr(),
                       ids, nf, frames.data_ptr() if frames is not None else None, _lib.stream_ptr())
     if check is not None:
         check.result()
-    object.__setattr__(data, "joint_pose_world", oMi.reshape(*batch, model.njoints, 7))
-    object.__setattr__(data, "joint_pose_local", liMi.reshape(*batch, model.njoints, 7))
+    object.__setattr__(data, "joint_pose_world", oMi)
+    object.__setattr__(data, "joint_pose_local", liMi)
     object.__setattr__(data, "joint_jacobians", None)
     if frames is not None:
         object.__setattr__(data, "frame_pose_world", frames.reshape(*batch, nf, 7))
@@ -172,9 +174,9 @@ def _jac_from_poses(model, data: Data, targets: Sequence[int], reference) -> tor
     out = torch.empty(B, len(targets), 6, model.nv, device=oMi.device, dtype=torch.float32)
     for s in range(0, len(targets), 64):
         chunk = list(targets[s:s + 64])
-        ids = (_lib.c_int32 * len(chunk))(*chunk)
+        ids = _lib.id_array(tuple(chunk))
         dst = out if len(targets) <= 64 else torch.empty(B, len(chunk), 6, model.nv, device=oMi.device)
-        with torch.cuda.device(oMi.device):
+        with _lib.on(oMi.device):
             _lib.call("br_frame_jacobians_from_poses", dt.ptr, of.data_ptr(), B, ids, len(chunk),
                       _ref_code(reference), dst.data_ptr(), _lib.stream_ptr())
         if dst is not out:
@@ -220,7 +222,7 @@ def frame_jacobians(model, q: torch.Tensor, frame_ids: Sequence[int], *,
     ``get_frame_jacobian`` for each id in ``frame_ids`` (at most 64), in one kernel.
     """
     _validate_q(model, q, check_quaternion)
-    frame_ids = [int(f) for f in frame_ids]
+    frame_ids = tuple(int(f) for f in frame_ids)
     if len(frame_ids) > 64:
         raise ShapeError("frame_jacobians takes at most 64 frames per call")
     batch = tuple(q.shape[:-1])
@@ -228,23 +230,19 @@ def frame_jacobians(model, q: torch.Tensor, frame_ids: Sequence[int], *,
     B = qf.shape[0]
     F = len(frame_ids)
     dt = device_tree(model, q.device)
-    J = torch.empty(B, F, 6, model.nv, device=q.device, dtype=torch.float32)
-    T = torch.empty(B, F, 7, device=q.device, dtype=torch.float32) if return_poses else None
-    ids = (_lib.c_int32 * F)(*frame_ids)
-    with torch.cuda.device(q.device):
-        _lib.call("br_frame_jacobians", dt.ptr, qf.data_ptr(), B, ids, F, _ref_code(reference),
+    J = torch.empty((*batch, F, 6, model.nv), device=q.device, dtype=torch.float32)
+    T = torch.empty((*batch, F, 7), device=q.device, dtype=torch.float32) if return_poses else None
+    with _lib.on(q.device):
+        _lib.call("br_frame_jacobians", dt.ptr, qf.data_ptr(), B, _lib.id_array(frame_ids), F, _ref_code(reference),
                   T.data_ptr() if T is not None else None, J.data_ptr(), _lib.stream_ptr())
-    J = J.reshape(*batch, F, 6, model.nv)
-    if T is None:
-        return J
-    return T.reshape(*batch, F, 7), J
+    return J if T is None else (T, J)
 
 
 def frame_jacobians_into(model, q: torch.Tensor, frame_ids, poses_out, jac_out, reference="local_world_aligned",
                          stream=None) -> None:
     """Allocation-free variant of ``frame_jacobians`` writing into caller buffers (for graphs / benchmarks)."""
     dt = device_tree(model, q.device)
-    ids = (_lib.c_int32 * len(frame_ids))(*[int(f) for f in frame_ids])
+    ids = _lib.id_array(tuple(int(f) for f in frame_ids))
     _lib.call("br_frame_jacobians", dt.ptr, q.data_ptr(), q.shape[0], ids, len(frame_ids), _ref_code(reference),
               poses_out.data_ptr() if poses_out is not None else None, jac_out.data_ptr(),
               stream if stream is not None else _lib.stream_ptr())

@@ -12,6 +12,7 @@ the forward primitives of the kernels (gradients of FK losses come from
 from __future__ import annotations
 
 import ctypes
+import math
 
 import torch
 
@@ -49,9 +50,9 @@ def _split(t: torch.Tensor, n: int, name: str) -> tuple[int, ...]:
 
 def _flat(t: torch.Tensor, batch: tuple[int, ...], own: tuple[int, ...], n: int) -> tuple[torch.Tensor, int]:
     """(contiguous (N, n) tensor, count), count 1 when ``t`` holds one element that broadcasts."""
-    numel = 1
-    for s in own:
-        numel *= s
+    numel = math.prod(own)
+    if own == batch and t.is_contiguous():
+        return t, numel
     if numel == 1:
         return t.reshape(1, n).contiguous(), 1
     e = t.reshape(*own, n).expand(*batch, n)
@@ -61,7 +62,7 @@ def _flat(t: torch.Tensor, batch: tuple[int, ...], own: tuple[int, ...], n: int)
 def apply(name: str, a: torch.Tensor, b: torch.Tensor | None = None) -> torch.Tensor:
     """``out = op(a, b)`` elementwise over the broadcast batch."""
     op = OPS[name]
-    na_f, nb_f, no_f = _sizes(op)
+    na_f, nb_f, no_f = _SIZES.get(op) or _sizes(op)
     ba = _split(a, na_f, "a")
     if nb_f:
         if b is None:
@@ -69,19 +70,17 @@ def apply(name: str, a: torch.Tensor, b: torch.Tensor | None = None) -> torch.Te
         bb = _split(b, nb_f, "b")
         if b.device != a.device:
             raise ShapeError("operands are on different devices")
-        batch = tuple(torch.broadcast_shapes(ba, bb))
+        batch = ba if ba == bb else tuple(torch.broadcast_shapes(ba, bb))
     else:
         bb, batch = (), ba
-    n = 1
-    for s in batch:
-        n *= s
+    n = math.prod(batch)
     af, na = _flat(a, batch, ba, na_f)
     bf, nb = _flat(b, batch, bb, nb_f) if nb_f else (None, 0)
-    out = torch.empty(n, no_f, device=a.device, dtype=torch.float32)
-    with torch.cuda.device(a.device):
+    out = torch.empty((*batch, *_SHAPE.get(no_f, (no_f,))), device=a.device, dtype=torch.float32)
+    with _lib.on(a.device):
         _lib.call("br_lie_op", op, af.data_ptr(), na, bf.data_ptr() if bf is not None else None, nb,
                   out.data_ptr(), n, _lib.stream_ptr())
-    return out.reshape(*batch, *_SHAPE.get(no_f, (no_f,)))
+    return out
 
 
 def se3_compose(a, b): return apply("se3_compose", a, b)            # noqa: E704

@@ -86,7 +86,7 @@ def solve_trajopt_batched(model, frame_id: int, goal: torch.Tensor, initial_q_tr
     start_c = start.contiguous().float() if start is not None else None
     ref_c = q_ref.contiguous().float() if q_ref is not None else None
     dt = device_tree(model, dev)
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         _lib.call("br_trajopt_solve", dt.ptr, int(frame_id), N, T, x0.data_ptr(),
                   ref_c.data_ptr() if ref_c is not None else None, goal_c.data_ptr(),
                   start_c.data_ptr() if start_c is not None else None, settings_from(cfg), x.data_ptr(),

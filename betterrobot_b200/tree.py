@@ -219,15 +219,22 @@ def _weak(model):
 _CACHE: dict[tuple[int, str], DeviceTree] = {}
 
 
+_NAMES: dict[torch.device, str] = {}
+
+
 def _drop(key) -> None:
     _CACHE.pop(key, None)
 
 
 def device_tree(model, device) -> DeviceTree:
-    device = torch.device(device)
+    if not isinstance(device, torch.device):
+        device = torch.device(device)
     if device.type == "cuda" and device.index is None:
         device = torch.device("cuda", torch.cuda.current_device())
-    key = (id(model), str(device))
+    name = _NAMES.get(device)
+    if name is None:
+        name = _NAMES[device] = str(device)
+    key = (id(model), name)
     dt = _CACHE.get(key)
     if dt is None or dt.model is not model:
         dt = DeviceTree(model, device)
