@@ -13,12 +13,12 @@
 //
 // Layout: a warp owns a tile of 32 consecutive configurations.  Their rows of every
 // input are one contiguous slab, copied into the warp's shared memory with 16-byte
-// cp.async copies (all of a tile's copies in flight at once); the slots of the other kinds
+// cp.async copies (all of a tile's copies in flight at once; pointers that are not
+// 16-byte aligned are read 4 bytes at a time, kVec = false); the slots of the other kinds
 // (free-flyer, spherical, planar, unbounded) are then computed one configuration per lane (the float64 exp / log runs on 32 lanes at once),
-// and the output slab is written with float4 stores, each lane producing 4 consecutive
-// outputs.  Memory bound: 4 * (nq + nv + nq) bytes per configuration for integrate,
-// 4 * (nq + nq + nv) for difference.  Pointers that are not 16-byte aligned take the
-// same path with 4-byte loads and stores (kVec = false).
+// and the output slab is written 32 consecutive floats at a time, each from the one or two
+// staged floats that a table of the CTA names.  Memory bound: 4 * (nq + nv + nq) bytes per
+// configuration for integrate, 4 * (nq + nq + nv) for difference.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -39,15 +39,8 @@ struct JointOpParams {
 
 constexpr int kJointOpsWarps = 4;
 
-// Floats of shared memory one warp stages.  integrate: two input tiles (the next one is
-// copied while this one is computed).  difference: one input tile, whose q0 rows also take
-// the outputs of the joints computed per lane (a joint's nv outputs overwrite the first nv
-// of its own nq >= nv slots); a second tile would halve its warps per SM (its float64 logs
-// make it compute heavy: measured at 1 M humanoid configurations, 104 -> 162 us).
-__host__ __device__ inline int joint_ops_in_floats(int nq, int nv, bool diff) { return 32 * (diff ? 2 * nq : nq + nv); }
-__host__ __device__ inline int joint_ops_warp_floats(int nq, int nv, bool diff) {
-  return diff ? joint_ops_in_floats(nq, nv, diff) : 2 * joint_ops_in_floats(nq, nv, diff);
-}
+// Floats of shared memory one warp stages: both inputs' rows of a tile.
+__host__ __device__ inline int joint_ops_warp_floats(int nq, int nv, bool diff) { return 32 * (diff ? 2 * nq : nq + nv); }
 
 __device__ __forceinline__ DPose dpose7(const float* p) {
   return DPose{d3(p[0], p[1], p[2]), make_double4(p[3], p[4], p[5], p[6])};
@@ -64,7 +57,39 @@ __device__ __forceinline__ void slab_in(float* s, const float* __restrict__ g, i
   for (int i = done + lane; i < n; i += 32) s[i] = g[i];
 }
 
-template <bool kVec>
+// exp of a free-flyer's step, as dse3_exp with one sincos and one reciprocal root: with k = sin(th/2) / th,
+// (1 - cos th) / th^2 = 2 k^2 and (th - sin th) / th^3 = (1 - 2 k cos(th/2)) / th^2.
+__device__ __forceinline__ DPose step_exp(double3 v, double3 w) {
+  const double th2 = ddot(w, w);
+  double b, c, k, ch;
+  if (th2 < 1e-8) {
+    b = 0.5 - th2 / 24.0;
+    c = 1.0 / 6.0 - th2 / 120.0;
+    k = 0.5 - th2 / 48.0;
+    ch = 1.0 - 0.125 * th2;
+  } else {
+    const double r = rsqrt(th2);
+    double sh;
+    sincos(0.5 * (th2 * r), &sh, &ch);
+    k = sh * r;
+    b = 2.0 * k * k;
+    c = fma(-2.0 * k, ch, 1.0) * (r * r);
+  }
+  const double3 wv = dcross(w, v);
+  DPose T;
+  T.t = dadd(dadd(v, dscale(wv, b)), dscale(dcross(w, wv), c));
+  T.q = make_double4(k * w.x, k * w.y, k * w.z, ch);
+  return T;
+}
+
+constexpr uint32_t kNoTerm = 0xffffu;
+// Tiles per warp of a CTA.  The hardware deals out the CTAs, so that SMs that run ahead take more (a fixed
+// share per SM left them idle for a sixth of the time), and a CTA's tables are made while its first copies are in
+// flight.  Measured, integrate / difference of 999,999 humanoids: 1 tile 82 / 88 us, 2 83 / 85, 4 84 / 86, one
+// resident wave with all tiles 87 / 89; a copy of as many bytes takes 74.
+constexpr int kTilesPerWarp = 2;
+
+template <bool kVec, bool kDiff>
 __global__ void __launch_bounds__(32 * kJointOpsWarps) joint_ops_kernel(const br_tree_t tree,
                                                                         const int32_t* __restrict__ active,
                                                                         const JointOpParams p) {
@@ -77,6 +102,22 @@ __global__ void __launch_bounds__(32 * kJointOpsWarps) joint_ops_kernel(const br
   __shared__ int8_t ffk[BR_MAX_JOINTS];
   __shared__ int nff;
   const int nq = tree.nq, nv = tree.nv;
+  const int lb = kDiff ? nq : nv;  // floats per configuration of b
+  const int lo = kDiff ? nv : nq;  // floats per configuration of out
+  const int lane = threadIdx.x & 31;
+  const int warps = blockDim.x >> 5;
+  float* A = slabs + 32 * lo + (size_t)(threadIdx.x >> 5) * joint_ops_warp_floats(nq, nv, kDiff);
+  float* Bs = A + 32 * nq;
+  const int64_t tiles = (p.batch + 31) >> 5;
+  auto fetch = [&](int64_t tile) {  // the tile's rows of both inputs
+    const int64_t b = tile << 5;
+    const int c = p.batch - b < 32 ? (int)(p.batch - b) : 32;
+    slab_in<kVec>(A, p.a + b * nq, c * nq, lane);
+    slab_in<kVec>(Bs, p.b + b * lb, c * lb, lane);
+  };
+  // the first tile's copies run while the tables below are made
+  int64_t tile = (int64_t)blockIdx.x * (kTilesPerWarp * warps) + (threadIdx.x >> 5);
+  if (tile < tiles) fetch(tile);
   for (int k = threadIdx.x; k < nq; k += blockDim.x) vmap[k] = -1;
   for (int k = threadIdx.x; k < nv; k += blockDim.x) qmap[k] = -1;
   if (threadIdx.x == 0) nff = 0;
@@ -99,48 +140,36 @@ __global__ void __launch_bounds__(32 * kJointOpsWarps) joint_ops_kernel(const br
     }
   }
   __syncthreads();
-  const bool diff = p.diff != 0;
-  const int lane = threadIdx.x & 31;
-  const int warps = blockDim.x >> 5;
-  const int lb = diff ? nq : nv;  // floats per configuration of b
-  const int lo = diff ? nv : nq;  // floats per configuration of out
-  const int IN = joint_ops_in_floats(nq, nv, diff);
-  float* base = slabs + (size_t)(threadIdx.x >> 5) * joint_ops_warp_floats(nq, nv, diff);
-  const bool dbl = kVec && !diff; // integrate with 16-byte copies: next tile in flight
-  const int64_t tiles = (p.batch + 31) >> 5;
-  const int64_t step = (int64_t)gridDim.x * warps;
+  // Output e of a tile is S[term e & 0xffff] (+ or -) S[term e >> 16] of the warp's slab S (both inputs' rows), the
+  // second left out where it is kNoTerm: 32 lanes at consecutive e read consecutive banks.  (Four outputs per lane as one
+  // float4, their slots found by division, took a 4-way bank conflict on every read.)
+  uint32_t* term = reinterpret_cast<uint32_t*>(slabs);
+  for (int e = threadIdx.x; e < 32 * lo; e += blockDim.x) {
+    const int c = e / lo, k = e - c * lo;
+    if (kDiff) {
+      const int kq = qmap[k];
+      term[e] = kq >= 0 ? (uint32_t)(32 * nq + c * nq + kq) | (uint32_t)(c * nq + kq) << 16
+                        : (uint32_t)(c * nq - kq - 1) | kNoTerm << 16;
+    } else {
+      term[e] = (uint32_t)e | (vmap[k] >= 0 ? (uint32_t)(32 * nq + c * nv + vmap[k]) : kNoTerm) << 16;
+    }
+  }
+  __syncthreads();
   const int n_ff = nff;
-  auto fetch = [&](int64_t t, float* buf) {  // the tile's rows of both inputs into buf
-    const int64_t b = t << 5;
-    const int c = p.batch - b < 32 ? (int)(p.batch - b) : 32;
-    slab_in<kVec>(buf, p.a + b * nq, c * nq, lane);
-    slab_in<kVec>(buf + 32 * nq, p.b + b * lb, c * lb, lane);
-  };
-  int64_t tile = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5);
-  if (dbl && tile < tiles) fetch(tile, base);
-  if (dbl) cp_async_commit();
-  for (int k = 0; tile < tiles; tile += step, ++k) {
+  for (int i = 0; i < kTilesPerWarp && tile < tiles; ++i, tile += warps) {
     const int64_t b0 = tile << 5;
     const int cnt = p.batch - b0 < 32 ? (int)(p.batch - b0) : 32;
-    float* A = dbl ? base + (k & 1) * IN : base;
-    float* Bs = A + 32 * nq;
-    if (dbl) {  // the next tile's copies are issued before this one is computed
-      if (tile + step < tiles) fetch(tile + step, base + ((k + 1) & 1) * IN);
-      cp_async_commit();
-      cp_async_wait_groups<1>();
-    } else {
-      fetch(tile, A);
-      if (kVec) cp_async_wait_all();
-    }
+    if (i > 0) fetch(tile);
+    if (kVec) cp_async_wait_all();
     __syncwarp();
     if (lane < cnt) {
       for (int f = 0; f < n_ff; ++f) {
         const int iq = ffq[f], iv = ffv[f], jt = ffk[f];
         float* qa = A + lane * nq + iq;
-        if (!diff) {
+        if (!kDiff) {
           const float* v = Bs + lane * nv + iv;
           if (jt == BR_JOINT_FREE_FLYER) {
-            DPose n = dcompose(dpose7(qa), dse3_exp(d3(v[0], v[1], v[2]), d3(v[3], v[4], v[5])));
+            DPose n = dcompose(dpose7(qa), step_exp(d3(v[0], v[1], v[2]), d3(v[3], v[4], v[5])));
             n.q = dqnormalize(n.q);
             qa[0] = (float)n.t.x; qa[1] = (float)n.t.y; qa[2] = (float)n.t.z;
             qa[3] = (float)n.q.x; qa[4] = (float)n.q.y; qa[5] = (float)n.q.z; qa[6] = (float)n.q.w;
@@ -185,40 +214,18 @@ __global__ void __launch_bounds__(32 * kJointOpsWarps) joint_ops_kernel(const br
       }
     }
     __syncwarp();
-    // out[e] for the tile's slab: 1:1 slots from the staged inputs, the other slots from above
     float* go = p.out + b0 * lo;
     const int n = cnt * lo;
-    auto val = [&](int c, int k) -> float {
-      if (!diff) {
-        const int kv = vmap[k];
-        const float x = A[c * nq + k];
-        return kv >= 0 ? x + Bs[c * nv + kv] : x;
-      }
-      const int kq = qmap[k];
-      return kq >= 0 ? Bs[c * nq + kq] - A[c * nq + kq] : A[c * nq - kq - 1];
-    };
-    int done = 0;
-    if (kVec) {
-      const int n4 = n >> 2;
-      for (int i = lane; i < n4; i += 32) {
-        int c = (4 * i) / lo, k = 4 * i - c * lo;
-        float r[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          r[u] = val(c, k);
-          if (++k == lo) { k = 0; ++c; }
-        }
-        reinterpret_cast<float4*>(go)[i] = make_float4(r[0], r[1], r[2], r[3]);
-      }
-      done = n4 << 2;
+#pragma unroll 4
+    for (int e = lane; e < n; e += 32) {
+      const uint32_t t = term[e];
+      float x = A[t & 0xffffu];
+      const uint32_t y = t >> 16;
+      if (y != kNoTerm) x = kDiff ? x - A[y] : x + A[y];
+      go[e] = x;
     }
-    for (int e = done + lane; e < n; e += 32) {
-      const int c = e / lo;
-      go[e] = val(c, e - c * lo);
-    }
-    __syncwarp();  // this tile's buffer is free for the tiles after the next
+    __syncwarp();  // the slab is free for the next tile
   }
-  if (kVec) cp_async_wait_all();
 }
 
 // *flag = 1 if any row's quaternion norm is further than tol from 1 (a NaN norm is not).  One pass over
@@ -267,23 +274,22 @@ extern "C" int br_configuration_op(const br_tree_t* tree, const int32_t* active_
   JointOpParams p = {a, b, out, batch, n_active, op == BR_OP_DIFFERENCE};
   const DeviceInfo& d = device_info();
   const bool vec = aligned16(a) && aligned16(b) && aligned16(out);
-  const size_t bytes = (size_t)kJointOpsWarps * joint_ops_warp_floats(tree->nq, tree->nv, p.diff) * sizeof(float);
+  const int lo = p.diff ? tree->nv : tree->nq;
+  const size_t bytes =
+      (32 * (size_t)lo + (size_t)kJointOpsWarps * joint_ops_warp_floats(tree->nq, tree->nv, p.diff)) * sizeof(float);
   if ((int64_t)bytes > d.max_smem_optin) return BR_ETOOBIG;
-  auto kern = vec ? joint_ops_kernel<true> : joint_ops_kernel<false>;
-  static size_t configured[2][16] = {};
-  size_t& have = configured[vec][d.device & 15];
+  auto kern = p.diff ? (vec ? joint_ops_kernel<true, true> : joint_ops_kernel<false, true>)
+                     : (vec ? joint_ops_kernel<true, false> : joint_ops_kernel<false, false>);
+  static size_t configured[4][16] = {};
+  size_t& have = configured[2 * p.diff + vec][d.device & 15];
   if (bytes > have) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return (int)e;
     have = bytes;
   }
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kJointOpsWarps, bytes);
-  if (per_sm < 1) per_sm = 1;
   const int64_t tiles = (batch + 31) / 32;
-  int64_t blocks = (tiles + kJointOpsWarps - 1) / kJointOpsWarps;
-  const int64_t cap = (int64_t)per_sm * d.sms;  // persistent: one wave, then grid-stride over tiles
-  if (blocks > cap) blocks = cap;
+  const int64_t blocks = (tiles + kTilesPerWarp * kJointOpsWarps - 1) / (kTilesPerWarp * kJointOpsWarps);
+  if (blocks > 0x7fffffff) return BR_ETOOBIG;
   kern<<<(unsigned)blocks, 32 * kJointOpsWarps, bytes, (cudaStream_t)stream>>>(*tree, active_joints, p);
   return (int)cudaGetLastError();
 }
