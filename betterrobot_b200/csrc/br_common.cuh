@@ -33,9 +33,6 @@ template <int N>
 __device__ __forceinline__ void bulk_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;" :: "n"(N) : "memory");
 }
-// Wait until every committed bulk group has completed (writes performed).
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
 // ---- cp.async (16-byte global -> shared copies that do not pass through registers) ----
 __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
   const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(sdst));
