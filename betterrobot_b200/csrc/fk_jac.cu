@@ -230,6 +230,20 @@ __device__ __forceinline__ void jac_column(const float* wcA, const float* wpT, c
   dst[3 * nv] = ang.x; dst[4 * nv] = ang.y; dst[5 * nv] = ang.z;
 }
 
+// a * b as compose, with the product that is rounded on its own in each quaternion component written out: left to
+// the compiler it follows the surrounding code, and the kernels of this file would differ in the last bit of a
+// placement (an IK problem whose target is such a placement can then take another number of iterations).
+__device__ __forceinline__ Pose compose_rn(const Pose& a, const Pose& b) {
+  const float4 p = a.q, q = b.q;
+  Pose c;
+  c.t = add(a.t, qrot(p, b.t));
+  c.q.x = fmaf(-p.z, q.y, fmaf(p.y, q.z, fmaf(p.w, q.x, __fmul_rn(p.x, q.w))));
+  c.q.y = fmaf(p.z, q.x, fmaf(p.y, q.w, fmaf(p.w, q.y, -__fmul_rn(p.x, q.z))));
+  c.q.z = fmaf(p.z, q.w, fmaf(-p.y, q.x, fmaf(p.x, q.y, __fmul_rn(p.w, q.z))));
+  c.q.w = fmaf(-p.z, q.z, fmaf(-p.y, q.y, fmaf(p.w, q.w, -__fmul_rn(p.x, q.x))));
+  return c;
+}
+
 template <int kRef, bool kFromQ>
 __global__ void fk_jac_kernel(const br_tree_t tree, const FkParams p) {
   extern __shared__ __align__(16) float smem[];
@@ -353,7 +367,7 @@ __global__ void fk_jac_kernel(const br_tree_t tree, const FkParams p) {
         for (int k = 0; k < 2; ++k) {
           const int j = lane + kWarp * k;
           if (j < nj && anc[k] >= 0) {
-            T[k] = compose(A[k], T[k]);
+            T[k] = compose_rn(A[k], T[k]);
             anc[k] = aa[k];
             store_split(wpT, wpQ, j, T[k]);
             wanc[j] = anc[k];
@@ -392,7 +406,7 @@ __global__ void fk_jac_kernel(const br_tree_t tree, const FkParams p) {
 
     // ---- target placements and world Jacobian columns --------------------
     for (int s = lane; s < nt; s += kWarp) {
-      const Pose Tt = compose(load_split(wpT, wpQ, s_tparent[s]), load_pose8(s_tplace + 8 * s));
+      const Pose Tt = compose_rn(load_split(wpT, wpQ, s_tparent[s]), load_pose8(s_tplace + 8 * s));
       store_pose8(wtgt + 8 * s, Tt);
       if (p.outputs & OUT_TPOSE) store_pose7(sT + 7 * s, Tt);
     }
@@ -576,7 +590,7 @@ __global__ void __launch_bounds__(256, kJac ? 2 : 3) fk_group_kernel(const br_tr
     for (int r = 0; r < rounds; ++r) {
       const int a = (int)(ancs >> (8 * r)) & 0xff;
       const Pose P = from_lane(T, a & 31);
-      if (a != 0xff) T = compose(P, T);
+      if (a != 0xff) T = compose_rn(P, T);
     }
     if (lane == 0) bulk_wait_read_all();  // the last group's blocks have been read out
     __syncwarp();
@@ -584,7 +598,7 @@ __global__ void __launch_bounds__(256, kJac ? 2 : 3) fk_group_kernel(const br_tr
     if ((p.outputs & OUT_OMI) && joint) store_pose7(sOMi + 7 * (sub_ * nj + own), T);
     for (int t0 = 0; t0 < nt; t0 += kG) {
       const int t = t0 + own < nt ? t0 + own : nt - 1;
-      const Pose Tt = compose(from_lane(T, base + s_tparent[t]), load_pose8(s_tplace + 8 * t));
+      const Pose Tt = compose_rn(from_lane(T, base + s_tparent[t]), load_pose8(s_tplace + 8 * t));
       if (t0 + own < nt) {
         if (kJac) store_pose8(wtgt + 8 * t, Tt);
         if (p.outputs & OUT_TPOSE) store_pose7(sT + 7 * (sub_ * nt + t), Tt);

@@ -54,3 +54,16 @@ def test_jacobians_beyond_l2():
         t, j = br.frame_jacobians(m, q[rows], ids)
         assert (T[rows] - t).abs().max() <= 2e-5
         _jac_close(J[rows].cpu().numpy(), j.cpu().numpy(), 2.0)
+
+
+@pytest.mark.parametrize("reference", ["world", "local_world_aligned", "local"])
+def test_kernels_agree_to_the_bit(reference):
+    """A batch whose Jacobians exceed L2 (staged records) against its rows in a small one (registers): the same
+    bits, so that a problem made from a placement does not depend on the batch it was computed in."""
+    m = syn.model_from_spec(syn.humanoid_spec())
+    ids = syn.op_frame_ids(m)
+    B = 2 * torch.cuda.get_device_properties(0).L2_cache_size // (len(ids) * 6 * m.nv * 4)
+    q = syn.random_q(m, B, 4).float().cuda()
+    T, J = br.frame_jacobians(m, q, ids, reference=reference)
+    t, j = br.frame_jacobians(m, q[:513], ids, reference=reference)
+    assert torch.equal(T[:513], t) and torch.equal(J[:513], j)
