@@ -216,7 +216,11 @@ class PackedIK:
                 ("q_rest", q_total if host_rest else 0, torch.float32, (q_total,))):
             self._sections[name] = (o, n, dtype, shape)
             o += (n + 3) & ~3
-        host = np.zeros(o, np.int32)
+        # staged in pinned memory (the allocator holds it until the copy has run); a capture refuses the copy
+        # of pageable memory, whose address a replay would read
+        capturing = torch.cuda.is_current_stream_capturing()
+        staged = torch.zeros(o, dtype=torch.int32, pin_memory=not capturing)
+        host = staged.numpy()
 
         def part(name, dtype=np.int32):
             o, n = self._sections[name][:2]
@@ -264,7 +268,7 @@ class PackedIK:
             qr = part("q_rest", np.float32)
             for c, m in enumerate(models):
                 qr[x0s[c]:x0s[c + 1]].reshape(-1, m.nq)[...] = rest[c].expand(self.counts[c], m.nq).numpy()
-        self._tables = torch.from_numpy(host).to(dev, non_blocking=True)
+        self._tables = staged.to(dev, non_blocking=not capturing)
         if not host_rest:
             self.q_rest = torch.empty(q_total, device=dev)
             for c, m in enumerate(models):
