@@ -753,8 +753,9 @@ __global__ void __launch_bounds__(256, 2) pose_loss_lanes_kernel(const br_tree_t
     if (__any_sync(0xffffffffu, far)) {             // joint angles of thousands of turns
       for (int k = 0; k < nvis; ++k) {
         const int4 m = meta_of(k);
+        if (!((m.x >> 16) & kLaneRevZ)) continue;   // (a fixed joint's idx_q may lie one past the row)
         const float x = gq[(lane < last ? lane : last) * nq + m.y];
-        if (((m.x >> 16) & kLaneRevZ) && fabsf(x) > kSincosHalfMax) {
+        if (fabsf(x) > kSincosHalfMax) {
           float sn, cs;
           sincosf(0.5f * x, &sn, &cs);
           qrow[m.y] = sn * rec[32 * k + kRecPlace + 3];
