@@ -167,11 +167,15 @@ class PackedIK:
                  with_residual: bool = False, target_kinds: Sequence | None = None):
         self._build(models, frame_ids, n_targets, q_rest, team_sizes, device, warps_per_cta, with_residual,
                     target_kinds, True)
+        # The tables hold the indices and offsets that the kernel addresses memory with, and a plan may be
+        # solved on any stream: the upload, queued on the current one, is complete when the plan is handed out.
+        torch.cuda.current_stream(self.device).synchronize()
 
     def _build(self, models, frame_ids, n_targets, q_rest, team_sizes, device, warps_per_cta, with_residual,
                target_kinds, fill: bool) -> None:
-        """``fill``: the identity targets and zero start configurations of a plan that is solved before
-        ``set_inputs`` are written."""
+        """Lay out and upload the plan, on the current stream and without waiting for it.  ``fill``: the
+        identity targets and zero start configurations of a plan that is solved before ``set_inputs``
+        are written."""
         if not 1 <= len(models) <= MAX_CLASSES:
             raise ShapeError(f"1..{MAX_CLASSES} robot classes per launch, got {len(models)}")
         self.device = torch.device(device)
