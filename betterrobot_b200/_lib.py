@@ -155,6 +155,12 @@ def on(device):
     return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
+def capturing(device) -> bool:
+    """Whether the stream that is current on ``device`` (not: on the current device) is being captured."""
+    with on(device):
+        return torch.cuda.is_current_stream_capturing()
+
+
 def stream_ptr(device=None) -> int:
     index = None if device is None else torch.device(device).index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)

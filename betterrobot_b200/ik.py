@@ -222,7 +222,7 @@ class PackedIK:
             o += (n + 3) & ~3
         # staged in pinned memory (the allocator holds it until the copy has run); a capture refuses the copy
         # of pageable memory, whose address a replay would read
-        capturing = torch.cuda.is_current_stream_capturing()
+        capturing = _lib.capturing(self.device)
         staged = torch.zeros(o, dtype=torch.int32, pin_memory=not capturing)
         host = staged.numpy()
 
