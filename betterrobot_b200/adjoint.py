@@ -31,9 +31,11 @@ from .tree import device_tree
 def path_slots(arrays, frame_ids: tuple) -> int:
     """Most joints on one root-to-leaf path that hold a waiting wrench in the adjoint's walk: in the tree
     pruned to the frames' ancestors, those with a child and a frame of their own or a second child.
-    Kept with the tree table, per frame set."""
+    Kept with the tree table, per frame set; -1 (not known) for a list that the entry point refuses."""
     n = arrays.path_slots.get(frame_ids)
     if n is None:
+        if not frame_ids or min(frame_ids) < 0 or max(frame_ids) >= arrays.nf:
+            return -1
         framed = {int(arrays.frame_parent[f]) for f in frame_ids}
         support = [int(x) for x in arrays.support]
         need = 0
