@@ -957,7 +957,8 @@ __global__ void __launch_bounds__(256) scale_rows_kernel(const float* __restrict
 //   warp kernel's time starts at 7 us and grows with the batch (loss and gradient in one pass, humanoid:
 //   12.6 us at 4,096, 21.6 at 8,192, 41 at 16,384; chain: 7.3 / 12 / 20 us at 1,300 / 4,096 / 8,192).
 //   The lines cross near 200 (njoints + nf) configurations, for the loss alone too.
-constexpr int kLanesNo = 1, kLanesMinWarps = 4, kLanesBatch = 200;
+constexpr int kLanesMinWarps = 4, kLanesBatch = 200;
+constexpr int kLanesNo = INT32_MIN;                 // neither a BR_E* code nor a cudaError_t
 constexpr int kLanesStatic = 1536;                  // static shared memory of the lane kernel, rounded up
 
 template <bool kGrad>
