@@ -47,6 +47,8 @@ template <bool> static void pose_loss_lanes_kernel() {}
 _TAIL = r"""
 extern "C" void fake_reset(int fail) { fail_attribute_call = fail; attribute_calls = 0; for (int& n : launches) n = 0; }
 extern "C" int fake_launches(int which) { return launches[which]; }
+extern "C" int static_bytes() { return (int)sizeof(br::LaneTables); }
+extern "C" int static_reserve() { return br::kLanesStatic; }
 """
 
 
@@ -59,7 +61,7 @@ def host(tmp_path_factory):
         return src[src.index(a):src.index(b, src.index(a))]
 
     layouts = between("struct LossParams", "template <bool kBackward>") + \
-        between("struct LaneLayout", "// A visit record")
+        between("struct LaneLayout", "// A visit record") + between("struct LaneTables", "template <bool kGrad>")
     code = src[src.index("// When the lane kernel is taken"):]
     which = iter(range(4))  # the lane kernel's launch, the warp kernel's, the scaling's two
     code = re.sub(r"\w+(?:<\w+>)?<<<.*?>>>\(.*?\);", lambda _: f"++launches[{next(which)}];", code)
@@ -96,3 +98,12 @@ def test_small_batches_take_the_warp_kernel(host):
     for name, call in _calls(host, 8_799).items():
         host.fake_reset(0)
         assert call() == 0 and (host.fake_launches(0), host.fake_launches(1)) == (0, 1), name
+
+
+def test_static_shared_memory_is_reserved(host):
+    """The host's fit against the opt-in limit counts all of the kernel's static arrays, and they are all in one struct."""
+    src = open(os.path.join(REPO, "betterrobot_b200", "csrc", "fk_adjoint.cu")).read()
+    kernel = src[src.index("pose_loss_lanes_kernel(const br_tree_t tree"):src.index("// out[b, :] = unit[b, :]")]
+    declared = re.findall(r"(?<!extern )__shared__ (\w+) (\w+);", kernel)
+    assert declared == [("LaneTables", "tab")] and kernel.count("__shared__") == 2   # it, and the dynamic slab
+    assert host.static_bytes() <= host.static_reserve()
