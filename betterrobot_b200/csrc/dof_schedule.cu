@@ -105,6 +105,9 @@ extern "C" int64_t br_dof_schedule(const int32_t* dof_parent, int32_t nv, uint32
   }
   for (int k = 0; k < nv; ++k)
     if (last[k] >= 0) tasks[4 * last[k] + 3] = (uint32_t)k + 1;
+  // the last further contribution is no contribution but the mark of a table with a row section, and the
+  // table's length (filled in below)
+  extras.insert(extras.end(), {BR_DOF_SCHED_MARK, 0u});
   const int64_t toff = ((5 + (int64_t)levels) + 3) & ~(int64_t)3;
   const int64_t entry_words = toff + (int64_t)tasks.size() + (int64_t)extras.size();
 
@@ -172,6 +175,7 @@ extern "C" int64_t br_dof_schedule(const int32_t* dof_parent, int32_t nv, uint32
   rstarts.push_back((uint32_t)(rtasks.size() / 4));
   const int64_t roff = (entry_words + 3) & ~(int64_t)3, rtoff = roff + toff;
   const int64_t words = rtoff + (int64_t)(rtasks.size() + rextras.size() + trunk_from.size());
+  extras.back() = (uint32_t)words;
   if (out && capacity >= words) {
     std::fill(out, out + toff, 0u);
     out[0] = (uint32_t)levels;

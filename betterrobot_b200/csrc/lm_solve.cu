@@ -390,12 +390,13 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
   // level schedule (br_tree_t.dof_sched): every offset it holds must address this
   // problem's factor storage; checked once per team and schedule
   const uint32_t* sched = tree.dof_sched;  // non-null: checked on the host
-  const uint32_t* rsched = sched + (((((5 + (int)sched[0] + 3) & ~3) + 4 * (int)sched[1] + 2 * (int)sched[2]) + 3) & ~3);
+  const int roff = ((((5 + (int)sched[0] + 3) & ~3) + 4 * (int)sched[1] + 2 * (int)sched[2]) + 3) & ~3;
+  const uint32_t* rsched = sched + roff;
   if (sched != sched_ok && !misc[0]) {
-    int lim = nv;                                      // the entry schedule's offsets: unpadded rows, then nv slots
+    int words = 0, lim = nv;                           // the entry schedule's offsets: unpadded rows, then nv slots
     for (int c = 0; c < nv; ++c) lim += ddep[c] + 1;
     const int nlev = (int)sched[0], ntask = (int)sched[1], nextra = (int)sched[2];
-    bool bad = nlev < 0 || nlev > nv || ntask < 0 || nextra < 0 || (int)sched[3] != misc[1];
+    bool bad = nlev < 0 || nlev > nv || ntask < 0 || nextra < 1 || (int)sched[3] != misc[1];
     auto starts_ok = [&](const uint32_t* st, int levs, int last) {
       bool ok = true;
 #pragma unroll 1
@@ -415,18 +416,23 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
       for (int p = tl; p < ntask; p += T) {
         const uint4 t4 = tk[p];
         bad |= (int)(t4.x & 0xffff) >= lim || (int)(t4.y & 0xffff) >= lim || (int)(t4.y >> 16) >= lim ||
-               (int)(t4.z & 0xffff) >= nv || (int)(t4.z >> 16) + (int)(t4.x >> 16) > nextra || (int)t4.w > nv;
+               (int)(t4.z & 0xffff) >= nv || (int)(t4.z >> 16) + (int)(t4.x >> 16) >= nextra || (int)t4.w > nv;
       }
 #pragma unroll 4
-      for (int e = tl; e < nextra; e += T) {
+      for (int e = tl; e < nextra - 1; e += T) {
         const uint2 e2 = ex[e];
         bad |= (int)(e2.x & 0xffff) >= lim || (int)(e2.x >> 16) >= lim || (int)e2.y >= nv;
       }
+      // a table of an older library ends with its contributions: no mark, and nothing to read behind them
+      const uint2 mark = ex[nextra - 1];
+      words = (int)mark.y;
+      bad |= mark.x != BR_DOF_SCHED_MARK || words < roff + ((5 + nlev + 3) & ~3);
     }
     if (!__any_sync(tm.mask, bad)) {                   // the row schedule: every pair inside the padded rows
       const int nr = rowoff[nv], nrt = (int)rsched[0], nrx = (int)rsched[1];
       const int blev = (int)(rsched[2] & 0xffff), ntr = (int)(rsched[2] >> 16);
-      bad = nrt < 0 || nrx < 0 || ntr > kTrunkMax || ntr > nv || blev + ntr != nlev || (int)rsched[3] != nr;
+      bad = nrt < 0 || nrx < 0 || ntr > kTrunkMax || ntr > nv || blev + ntr != nlev || (int)rsched[3] != nr ||
+            (int64_t)words != roff + ((5 + nlev + 3) & ~3) + 4ll * nrt + nrx + (ntr > 0 ? nv - ntr : 0);
       if (!bad) {
         bad |= !starts_ok(rsched + 4, blev, nrt);
         const uint32_t* rt = rsched + ((5 + nlev + 3) & ~3);

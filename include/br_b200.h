@@ -40,6 +40,7 @@ extern "C" {
 #define BR_MAX_NV 64
 #define BR_MAX_NQ 128
 #define BR_MAX_TARGETS 64   /* frames (or joints) per Jacobian launch            */
+#define BR_DOF_SCHED_MARK 0x5752ffffu /* no contribution's word: offsets are below 0xffff (br_dof_schedule) */
 
 /* ---- joint kinds in the tree table ----------------------------------- */
 #define BR_JOINT_FIXED 0        /* universe, fixed                                */
@@ -106,14 +107,16 @@ typedef struct br_tree {
  * on scheduling.  The right-hand side rides along as one extra slot per DOF (forward
  * substitution inside the factorization).
  *
- * Layout (uint32 words): [0] levels, [1] tasks, [2] extra contributions, [3] 1 + the
+ * Layout (uint32 words): [0] levels, [1] tasks, [2] extra contributions and one, [3] 1 + the
  * deepest DOF depth, [4 .. 4 + levels] first task of each level (the last = tasks),
  * then at word toff = roundup(5 + levels, 4) the tasks, 4 words each:
  *   {dst | (n_extra << 16), a | (b << 16), k | (first_extra << 16), f}
  *   dst -= m[a] * m[b] / (pivot_k + damp), then the same for each extra contribution;
  *   f = c + 1 when the task is the last update of DOF c's diagonal (its pivot is then
  *   final), else 0,
- * then at toff + 4 * tasks the extra contributions, 2 words each: {a | (b << 16), k}.
+ * then at toff + 4 * tasks the extra contributions, 2 words each: {a | (b << 16), k}, and after them
+ * {BR_DOF_SCHED_MARK, words of the whole table}: the LM refuses a table without this pair (one of a
+ * library that wrote no row schedule) or with another length, and reads nothing past the pair then.
  * Offsets index the packed rows (row c starts at sum_{c' < c} (depth(c') + 1), its
  * diagonal at depth(c)) followed by the nv right-hand-side slots.
  *
