@@ -7,14 +7,16 @@ In the reference its gradient comes from torch autograd through every SE3 op
 of the FK loop (``src/better_robot/kinematics/forward.py:79-81`` keeps that tape
 on purpose); here it is the hand-written adjoint of ``fk_adjoint.cu``.
 
-A configuration's loss depends on its own q only, so a forward pass whose ``q`` needs a gradient
-computes the loss and each configuration's own gradient together (one walk over the tree instead of
+A configuration's loss depends on its own q only, so a forward pass whose ``q`` needs a gradient can
+compute the loss and each configuration's own gradient together (one walk over the tree instead of
 one per pass); ``backward`` scales that gradient row by row with the incoming one.  Without a
 gradient to compute, the forward evaluates the loss alone.
 
-``mode`` ("store", "recompute" or "auto") chose between saving the joint placements and running the
-kinematics again in the backward.  The one-pass forward needs neither: every mode computes and
-returns the same.
+Modes: ``"store"`` does that, and keeps ``batch * nq`` floats for the backward; ``"recompute"`` evaluates the
+loss alone, keeps nothing of its own, and walks the tree again for the gradient in the backward (for
+when memory is short, or no backward may follow); ``"auto"`` is ``"store"``, the faster of the two with a
+backward at every batch (humanoid, 12 frames, kernels of both passes: 34 against 50 us at B = 16,384, 194
+against 320 at 262,144; forward alone 31 against 19, 176 against 103).
 """
 
 from __future__ import annotations
@@ -65,8 +67,11 @@ def _loss_only(model, q, frame_ids, targets, weights):
 
 class _PoseLoss(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, targets, weights, model, frame_ids, want_grad):
-        if not want_grad:
+    def forward(ctx, q, targets, weights, model, frame_ids, mode):
+        """``mode``: "store", "recompute", or None where no gradient can be asked for."""
+        if mode != "store":
+            ctx.model, ctx.frame_ids = model, frame_ids
+            ctx.save_for_backward(q, targets, weights)
             return _loss_only(model, q, frame_ids, targets, weights)
         loss = torch.empty(q.shape[0], device=q.device, dtype=torch.float32)
         unit = torch.empty_like(q)
@@ -81,14 +86,20 @@ class _PoseLoss(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_loss):
-        unit = ctx.saved_tensors[3]
+        q, targets, weights, *stored = ctx.saved_tensors
         g = grad_loss if grad_loss.dtype == torch.float32 else grad_loss.float()
-        if g.stride(0) not in (0, 1):
-            g = g.contiguous()
-        grad_q = torch.empty_like(unit)
-        with _lib.on(unit.device):
-            _lib.call("br_scale_rows", unit.data_ptr(), g.data_ptr(), g.stride(0), unit.shape[0], unit.shape[1],
-                      grad_q.data_ptr(), _lib.stream_ptr())
+        grad_q = torch.empty_like(q)
+        with _lib.on(q.device):
+            if stored:
+                if g.stride(0) not in (0, 1):
+                    g = g.contiguous()
+                _lib.call("br_scale_rows", stored[0].data_ptr(), g.data_ptr(), g.stride(0), q.shape[0], q.shape[1],
+                          grad_q.data_ptr(), _lib.stream_ptr())
+            else:
+                g = g.contiguous()
+                _lib.call("br_pose_loss_backward", device_tree(ctx.model, q.device).ptr, q.data_ptr(), None, q.shape[0],
+                          _lib.id_array(ctx.frame_ids), len(ctx.frame_ids), targets.data_ptr(), weights.data_ptr(),
+                          int(weights.dim() == 2), g.data_ptr(), grad_q.data_ptr(), _lib.stream_ptr())
         return grad_q, None, None, None, None, None
 
 
@@ -98,7 +109,7 @@ def pose_loss(model, q: torch.Tensor, frame_ids: Sequence[int], targets: torch.T
 
     The backward kernel maps gradients to raw q for every joint kind of the tree table
     (fixed, revolute, unbounded revolute, prismatic, free-flyer, spherical, planar,
-    translation).
+    translation).  ``mode``: "store", "recompute" or "auto", above.
     """
     _validate_q(model, q, check_quaternion)
     if q.dim() != 2:
@@ -111,6 +122,9 @@ def pose_loss(model, q: torch.Tensor, frame_ids: Sequence[int], targets: torch.T
         raise ShapeError(f"weights must be ({F},) or ({B}, {F}), got {tuple(weights.shape)}")
     if mode not in ("store", "recompute", "auto"):
         raise ValueError(f"mode must be 'store', 'recompute' or 'auto', got {mode!r}")
-    want_grad = torch.is_grad_enabled() and (q.requires_grad or targets.requires_grad or weights.requires_grad)
+    if not (torch.is_grad_enabled() and (q.requires_grad or targets.requires_grad or weights.requires_grad)):
+        mode = None
+    elif mode == "auto":
+        mode = "store"
     return _PoseLoss.apply(q.contiguous(), targets.contiguous().float(), weights.contiguous().float(), model,
-                           frame_ids, want_grad)
+                           frame_ids, mode)
