@@ -624,8 +624,7 @@ def bench_adjoint(steps: int, warmup: int):
             e1.record(stream)
             torch.cuda.synchronize()
             ms = e0.elapsed_time(e1) / steps
-            fl = adjoint_flops_per_config(m, fids, recompute=(mode == "recompute" or
-                                                              (mode == "auto" and B * m.njoints * 28 > 126 << 20)))
+            fl = adjoint_flops_per_config(m, fids, recompute=mode == "recompute")
             tf = B * fl / (ms * 1e-3) / 1e12
             out[f"B{B}_{mode}"] = {"ms_fwd_bwd": ms, "configs_per_s": B / (ms * 1e-3), "flops_per_config": fl,
                                    "tflops": tf, "frac_fp32_peak": tf / FP32_PEAK_TFLOPS}
