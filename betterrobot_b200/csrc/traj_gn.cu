@@ -150,6 +150,9 @@ __device__ __forceinline__ int tri_at(int r, int c) { return r * (r + 1) / 2 + c
 // (64 trajectories of 64 knots, six iterations, 256 against 128 threads: chain of 7 94 against 100 us,
 // 20 DOFs 144 / 160, humanoid 250 / 280; with more trajectories than SMs two CTAs of 128 run at once).
 
+// Threads that the terms of a block's sums are dealt to, whatever its own number.
+constexpr int kSumThreads = 256;
+
 // kManifold: the tree has joints whose configuration is not their tangent coordinates
 // (free-flyer, spherical, planar, unbounded revolute): knot differences and the retraction go
 // through Model.difference / Model.integrate; otherwise they are q1 - q0 and q + v.
@@ -253,16 +256,39 @@ __global__ void __launch_bounds__(kNT, 256 / kNT) traj_gn_kernel(const TrajParam
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
   };
-  // sum over the block; every thread gets the same value (the warps' partials are added in
-  // warp order by every thread)
-  auto block_sum = [&](double v) -> double {
-    v = warp_sum(v);
+  // Sum over the block; every thread gets the same value.  A trajectory's sums do not depend on the block
+  // that its launch chose: terms are dealt to kSumThreads threads, of which one of a smaller block stands
+  // for several (its terms in turn, Sum::add), and the warps' partials are added in the order of those.
+  constexpr int kParts = kSumThreads / NT;
+  struct Sum {
+    double v[kParts] = {};
+    int turn = 0;
+    __device__ __forceinline__ void add(double x) {
+      if (kParts == 1) {
+        v[0] += x;
+      } else {
+        const double s = (turn ? v[kParts - 1] : v[0]) + x;
+        if (turn) v[kParts - 1] = s;
+        else v[0] = s;
+        turn ^= 1;
+      }
+    }
+    __device__ __forceinline__ void next_loop() { turn = 0; }   // every loop deals from the first thread
+  };
+  static_assert(kParts <= 2, "Sum::add alternates between two");
+  auto block_sum = [&](const Sum& a) -> double {
+    double v[kParts];
+#pragma unroll
+    for (int h = 0; h < kParts; ++h) v[h] = warp_sum(a.v[h]);
     __syncthreads();                                  // the previous reduction's reads are done
-    if (lane == 0) red[warp] = v;
+    if (lane == 0) {
+#pragma unroll
+      for (int h = 0; h < kParts; ++h) red[h * NW + warp] = v[h];
+    }
     __syncthreads();
     double s = 0.0;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) s += red[w];
+    for (int w = 0; w < kSumThreads / kWarp; ++w) s += red[w];
     return s;
   };
   // float64 FK of knot t of trajectory `xs` by one warp (pose term h: buffers pA / pB + 8 nj h,
@@ -446,40 +472,42 @@ __global__ void __launch_bounds__(kNT, 256 / kNT) traj_gn_kernel(const TrajParam
   };
   // total cost 0.5 |r|^2 at xs (pose terms evaluated into rg / rs)
   auto cost_of = [&](const double* xs) -> double {
-    double acc = 0.0;
+    Sum acc;
     pose_terms(xs, false, false);
     if (kManifold) knot_differences(xs);
     for (int e = tid; e < (T - 2) * nv; e += NT) {              // smoothness.py:118-125
       const double a = kManifold ? c * (dd[e + nv] - dd[e]) : c * (xs[e + 2 * nv] - 2.0 * xs[e + nv] + xs[e]);
-      acc += a * a;
+      acc.add(a * a);
     }
+    acc.next_loop();
     if (kManifold) {
       for (int e = tid; e < nqT; e += NT) {                     // limits.py:56-62
         const int i = divq.mod(e);
         const double lo = fmax((double)lower[i] - xs[e], 0.0), hi = fmax(xs[e] - (double)upper[i], 0.0);
-        acc += wl * wl * (lo * lo + hi * hi);
+        acc.add(wl * wl * (lo * lo + hi * hi));
       }
-      for (int e = tid; e < n; e += NT) acc += wr * wr * dr[e] * dr[e];   // regularization.py:143-152
+      acc.next_loop();
+      for (int e = tid; e < n; e += NT) acc.add(wr * wr * dr[e] * dr[e]);   // regularization.py:143-152
     } else {                                                    // nq == nv: one pass for both
       for (int e = tid; e < n; e += NT) {
         const int i = divv.mod(e);
         const double lo = fmax((double)lower[i] - xs[e], 0.0), hi = fmax(xs[e] - (double)upper[i], 0.0);
         const double d = xs[e] - (double)xref[e];
-        acc += wl * wl * (lo * lo + hi * hi) + wr * wr * d * d;
+        acc.add(wl * wl * (lo * lo + hi * hi) + wr * wr * d * d);
       }
     }
-    acc = block_sum(acc);
+    const double knots = block_sum(acc);
     double pc = 0.0;
     for (int k = 0; k < 6; ++k) {
       if (has_goal) pc += wg * wg * rg[k] * rg[k];
       if (has_start) pc += ws * ws * rs[k] * rs[k];
     }
-    return 0.5 * (acc + pc);
+    return 0.5 * (knots + pc);
   };
   // pose Jacobians and g = J^T r at x; returns |g|
   auto build = [&]() -> double {
     pose_terms(x, true, true);                        // FK and xi of x from the cost evaluation of x
-    double gg = 0.0;
+    Sum gg;
     for (int e = tid; e < n; e += NT) {
       const int t = divv.div(e), i = e - t * nv;
       double acc = 0.0;
@@ -504,10 +532,9 @@ __global__ void __launch_bounds__(kNT, 256 / kNT) traj_gn_kernel(const TrajParam
       if (has_start && t == 0)
         for (int r = 0; r < 6; ++r) acc += ws * ws * Js[r * nv + i] * rs[r];
       g[e] = acc;
-      gg += acc * acc;
+      gg.add(acc * acc);
     }
-    gg = block_sum(gg);
-    return sqrt(gg);
+    return sqrt(block_sum(gg));
   };
   // bands of J^T J + damp I at x (DOF i): diagonal at knot t, H[(t+1,i),(t,i)], and
   // H[(t+2,i),(t,i)] = c2 for t <= T-3.  Acceleration row s has coefficients (1, -2, 1)
@@ -775,13 +802,10 @@ __global__ void __launch_bounds__(kNT, 256 / kNT) traj_gn_kernel(const TrajParam
         for (int e = tid; e < ne; e += NT) {
           const int2 rc = tri_decode(e);
           const double *lr = Sb + tri_at(k1 + rc.x, k0), *lc = Sb + tri_at(k1 + rc.y, k0);
-          double s0 = 0.0, s1 = 0.0;
+          double acc = 0.0;                                        // in the tiles' order
 #pragma unroll
-          for (int j = 0; j < kPan; j += 2) {
-            s0 += lr[j] * (lc[j] * sd[k0 + j]);
-            s1 += lr[j + 1] * (lc[j + 1] * sd[k0 + j + 1]);
-          }
-          Sb[tri_at(k1 + rc.x, k1 + rc.y)] -= s0 + s1;
+          for (int j = 0; j < kPan; ++j) acc += lr[j] * (lc[j] * sd[k0 + j]);
+          Sb[tri_at(k1 + rc.x, k1 + rc.y)] -= acc;
         }
       } else {
         const int nt = (nr + 3) >> 2;
