@@ -332,7 +332,7 @@ __device__ void solve_problem(const LmParams& P, const br_tree_t& tree, int prob
   // path; limit, rest and damping terms are diagonal), so J^T J is stored as one row per
   // DOF over its ancestors and itself, entry (i, j) at rowoff[i] + 1 + ddep[j] (the row's
   // first slot holds its right-hand side; rows have even lengths), and factors
-  // leaves first with no fill-in.  DOF numbering is topological (dpar[c] < c), so a
+  // leaves first with no fill-in.  DOF numbering is topological (a parent's index is smaller), so a
   // DOF's ancestors have smaller indices.
   // Lane c's ancestors are the DOFs of its joint's proper ancestors and the earlier DOFs of its own.
   tm.sync();

@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kNT, 256 / kNT) traj_gn_kernel(const TrajParam
   const int m = T - 2;
   const double h1 = -4.0 * c2;                        // H[(p+1), (p)] inside the interior
 
-  // Twisted elimination, two threads per DOF (for more DOFs than cyclic reduction has warps): thread 2i
+  // Twisted elimination, two threads per DOF (at least kTwistMin interior knots): thread 2i
   // takes rows 0..k-1 top-down (L D L^T), thread 2i + 1 rows m-1..k+2 bottom-up, k = m / 2, and both then
   // reduce the 2 x 2 block of rows k, k+1 from the two sides' updates.  The multipliers into the middle
   // block are kept in the free slots of rows k, k+1 (bl1), every second-neighbour multiplier is c2 times

@@ -292,6 +292,9 @@ BR_API int64_t br_lm_team_floats(const br_tree_t* tree, int32_t max_targets);
  * world joint placements [batch, njoints, 7] are stored for the backward pass
  * ("store" mode).  The reference evaluates this loss with its per-op torch FK
  * (src/better_robot/kinematics/forward.py:73-135, lie/se3.py log/compose).
+ * Without placements to store, batches of at least 200 (njoints + n_frames) configurations
+ * run another kernel than smaller ones (here and below): a configuration's loss and
+ * gradient then agree to float32 rounding with those of a smaller batch, not to the bit.
  */
 BR_API int br_pose_loss(const br_tree_t* tree, const float* q, int64_t batch, const int32_t* frame_ids,
                         int32_t n_frames, const float* targets, const float* weights, int32_t weights_per_config,
