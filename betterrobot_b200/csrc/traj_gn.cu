@@ -738,7 +738,8 @@ __global__ void __launch_bounds__(kNT, 256 / kNT) traj_gn_kernel(const TrajParam
     // L D L^T of S in panels of kPan columns: warp 0 eliminates the panel on its first 32 rows (lane r row
     // k0 + r; every lane carries the pivots, so that one reciprocal and one multiply-add separate two of
     // them), one thread per row the rows below, and the block updates the rest of S: one entry per thread
-    // while they are few, else 4 x 4 tiles.  The panel's entries stay as L; sdi 1 / pivot, sd pivot.
+    // while they are few, else 4 x 4 tiles (the same sums in the same order).  The panel's entries stay as L;
+    // sdi 1 / pivot, sd pivot.
     constexpr int kPan = 8;
     bool pos = true;
     for (int k0 = 0; k0 < nb; k0 += kPan) {
